@@ -1,7 +1,8 @@
 // Standalone quantize, in-place dequantize and low-rank factorisation kernels (sm_100a).
 //
-// Quantize and low-rank: one CTA of 256 threads per (row, value head), the head's 128 x 128 fp32 tile in shared memory for
-// the whole kernel.  Dequantize: persistent CTAs that walk the heads, each head's checkpoint staged in shared memory.
+// Quantize: persistent CTAs, a head's 128 x 128 fp32 tile in the registers of one CTA, the next head's on its way into shared
+// memory.  Dequantize: persistent CTAs that walk the heads, each head's checkpoint staged in shared memory.  Low-rank: one CTA
+// of 256 threads per matrix, which stays in shared memory.
 // Either way the in-place rewrite of a slot (fp32 state <-> packed 8-bit checkpoint) never reads what it has already
 // overwritten.
 #include "lq_linalg.cuh"
@@ -9,165 +10,431 @@
 namespace lq {
 
 // ------------------------------------------------------------------------------------------------------------------
-// shared pieces
+// quantize
 // ------------------------------------------------------------------------------------------------------------------
-// Row-wise INT8 stage.  The results are those of the reference's true divisions (leapquant/kernels.py:2218-2229):
-//   Sv[v] = max(max_c |E / Sk|, EPS),  code = clamp(rint(E / (Sk Sv) * 127)),
-// but a division is only executed where it can matter.  Row maximum: the candidates are found with |E| * (1 / Sk) (within
-// two ulp of the quotient), and only elements within 1e-6 of the best candidate are divided -- the true maximum is always
-// among them.  Codes: y = E * (1 / Sk) * (127 / Sv) is within 5e-5 code units of the exact value, so rint(y) is the exact
-// code unless y lies within 1e-3 of a half-integer, and only then is the reference's expression evaluated.
-// Warp w takes rows 16 w .. 16 w + 15, four rows per pass; eight lanes share a row, each lane owns columns
-// {32 i + 4 l8 .. + 3 | i = 0..3} so that the eight float4 reads of a row are one contiguous 128-B line.
-__device__ __forceinline__ void quant_rows_div(const float* __restrict__ E, const float* __restrict__ sk, const float* __restrict__ rsk,
-                                               char* base, int tid) {
-    const int warp = tid >> 5, lane = tid & 31, l8 = lane & 7, g = lane >> 3;
-    uint32_t* codes = reinterpret_cast<uint32_t*>(base + CK_CODES);
-    float* svg = reinterpret_cast<float*>(base + CK_SV);
+// One head = one 128 x 128 fp32 tile, held in REGISTERS by the 256 threads of a CTA (64 values each) from the moment it has
+// arrived until its codes are stored; persistent CTAs, two per SM.  The tile is read from shared memory once, so that the
+// buffer is free for the next head's 64 KB -- one bulk asynchronous copy, in flight during the whole of this head's
+// arithmetic -- and every product of the subspace iteration works on registers with packed f32x2 multiply-adds (two fp32
+// products per instruction, each rounded as the scalar one would be).
+// Thread (warp w, lane): lc = lane % 16, lr = lane / 16 owns rows 16 w + 8 lr + i (i < 8) and columns 4 lc .. + 3, 64 + 4 lc .. + 3.
+//   P = S^T Q: 8 rows are summed in the thread, two half-warps by one exchange, eight warps through shared memory.
+//   Q = S P:   8 columns in the thread, sixteen lanes by halving exchanges; a warp ends with its own 16 rows.
+// What bounds it: issue slots of the sixteen resident warps (R = 4: 14 400 warp instructions per head, a third of them the
+// multiply-adds, issued in 39 % of the cycles); the previous form read the tile from shared memory for every product (32 000
+// instructions per head, three CTAs per SM).  Dequantize + quantize of 8 192 GDN heads: 496 -> 390 us, of 416 heads 39 -> 36 us,
+// of 1 536 KDA heads (R = 8, three iterations) 277 -> 214 us.
+constexpr int QZ_TILE = 128 * 128 * 4;
+template <int R>
+__host__ __device__ constexpr int qz_smem_bytes() { return QZ_TILE + 8 * R * 128 * 4 + R * 128 * 4 + R * 128 * 8 + R * 128 * 4; }
+
+struct QzTile {
+    float2 s[8][4];                       // [row i][column pair]: pairs 0, 1 = columns 4 lc .. + 3; 2, 3 = 64 + 4 lc .. + 3
+};
+// partial products over the warp's 16 rows: part[w][r][c] = sum_row S[row][c] Q[row][r]; Qd: [128][R] values duplicated to pairs
+template <int R>
+__device__ __forceinline__ void qz_coldot(const QzTile& t, const float2* __restrict__ Qd, float* __restrict__ part, int warp, int lane) {
+    const int lc = lane & 15, lr = lane >> 4;
+    const float2* qrow = Qd + (16 * warp + 8 * lr) * R;
+    float* out = part + warp * (R * 128) + 64 * lr + 4 * lc;
 #pragma unroll 1
-    for (int it = 0; it < 4; ++it) {
-        const int row = warp * 16 + it * 4 + g;
-        float e[16], a[16];
-        float amax = 0.f;
+    for (int rb = 0; rb < R; rb += 4) {
+        float2 acc[4][4];                 // [column pair][r]
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 ev = *reinterpret_cast<const float4*>(E + row * LDB + i * 32 + l8 * 4);
-            const float4 rv = *reinterpret_cast<const float4*>(rsk + i * 32 + l8 * 4);
-            e[4 * i + 0] = ev.x; e[4 * i + 1] = ev.y; e[4 * i + 2] = ev.z; e[4 * i + 3] = ev.w;
-            a[4 * i + 0] = ev.x * rv.x; a[4 * i + 1] = ev.y * rv.y; a[4 * i + 2] = ev.z * rv.z; a[4 * i + 3] = ev.w * rv.w;
+        for (int i = 0; i < 8; ++i) {
+            const float4 qa = *reinterpret_cast<const float4*>(qrow + i * R + rb), qb = *reinterpret_cast<const float4*>(qrow + i * R + rb + 2);
+            const float2 q[4] = {make_float2(qa.x, qa.y), make_float2(qa.z, qa.w), make_float2(qb.x, qb.y), make_float2(qb.z, qb.w)};
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) acc[p][r] = i == 0 ? __fmul2_rn(t.s[i][p], q[r]) : __ffma2_rn(t.s[i][p], q[r], acc[p][r]);
         }
+        // the half-warp lr keeps the columns 64 lr + 4 lc .. + 3
 #pragma unroll
-        for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(a[i]));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-        const float thr = amax * (1.0f - 1e-6f);
-        float rmax = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (fabsf(a[i]) >= thr) rmax = fmaxf(rmax, fabsf(e[i] / sk[(i >> 2) * 32 + l8 * 4 + (i & 3)]));
-        rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, 1));
-        rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, 2));
-        rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, 4));
-        const float svv = fmaxf(rmax, EPS);
-        if (l8 == 0) svg[row] = svv;
-        const float rv127 = QMAX / svv;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            // rint() by adding 1.5 * 2^23: the sum's low mantissa byte is the code in two's complement.  |y| <= 127 (1 + 3e-7) by
-            // construction of Sv, so the reference's clamp to [-127, 127] never acts and is not evaluated.
-            uint32_t b[4];
+        for (int r = 0; r < 4; ++r) {
+            float v[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const float y = a[4 * i + k] * rv127;
-                float t = y + 12582912.0f;
-                const float c = t - 12582912.0f;
-                if (fabsf(fabsf(y - c) - 0.5f) < 1e-3f)                        // on a rounding boundary: the exact expression decides
-                    t = e[4 * i + k] / (sk[i * 32 + l8 * 4 + k] * svv) * QMAX + 12582912.0f;
-                b[k] = __float_as_uint(t);
+                const float2 lo = acc[k >> 1][r], hi = acc[2 + (k >> 1)][r];
+                const float a = (k & 1) ? lo.y : lo.x, b = (k & 1) ? hi.y : hi.x;
+                v[k] = (lr ? b : a) + __shfl_xor_sync(0xffffffffu, lr ? a : b, 16);
             }
-            codes[row * 32 + i * 8 + l8] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+            *reinterpret_cast<float4*>(out + (rb + r) * 128) = make_float4(v[0], v[1], v[2], v[3]);
         }
     }
 }
-
-// ------------------------------------------------------------------------------------------------------------------
-// quantize
-// ------------------------------------------------------------------------------------------------------------------
+// X[r][c] = sum over the eight warps' partials (all 256 threads), on request rounded to f16 values
 template <int R>
-__global__ void __launch_bounds__(NT_LA, 3)
+__device__ __forceinline__ void qz_sum_parts(const float* __restrict__ part, float* __restrict__ X, int tid, bool round16) {
+    constexpr int PT = R * 128 / NT_LA;   // outputs per thread: 2 or 4
+    float a[PT];
+#pragma unroll
+    for (int k = 0; k < PT; ++k) a[k] = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        if constexpr (PT == 2) {
+            const float2 v = *reinterpret_cast<const float2*>(part + w * (R * 128) + 2 * tid);
+            a[0] += v.x; a[1] += v.y;
+        } else {
+            const float4 v = *reinterpret_cast<const float4*>(part + w * (R * 128) + 4 * tid);
+            a[0] += v.x; a[1] += v.y; a[2] += v.z; a[3] += v.w;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < PT; ++k) X[PT * tid + k] = round16 ? round_f16(a[k]) : a[k];
+}
+// X[r][row] = sum_c S[row][c] P[r][c]
+template <int R>
+__device__ __forceinline__ void qz_rowdot(const QzTile& t, const float* __restrict__ P, float* __restrict__ X, int warp, int lane) {
+    const int lc = lane & 15, lr = lane >> 4;
+    const bool b3 = lc & 8, b2 = lc & 4, b1 = lc & 2, b0 = lc & 1;
+#pragma unroll 1
+    for (int rb = 0; rb < R; rb += 4) {
+        float v[4][4];                    // [row i or i + 4, by bit 3 of lc][r]
+        float2 pv[4][4];                  // [r][column pair]
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float4 lo = *reinterpret_cast<const float4*>(P + (rb + r) * 128 + 4 * lc), hi = *reinterpret_cast<const float4*>(P + (rb + r) * 128 + 64 + 4 * lc);
+            pv[r][0] = make_float2(lo.x, lo.y); pv[r][1] = make_float2(lo.z, lo.w);
+            pv[r][2] = make_float2(hi.x, hi.y); pv[r][3] = make_float2(hi.z, hi.w);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                float2 x = __fmul2_rn(t.s[i][0], pv[r][0]), y = __fmul2_rn(t.s[i + 4][0], pv[r][0]);
+#pragma unroll
+                for (int p = 1; p < 4; ++p) {
+                    x = __ffma2_rn(t.s[i][p], pv[r][p], x);
+                    y = __ffma2_rn(t.s[i + 4][p], pv[r][p], y);
+                }
+                const float xs = x.x + x.y, ys = y.x + y.y;
+                v[i][r] = (b3 ? ys : xs) + __shfl_xor_sync(0xffffffffu, b3 ? xs : ys, 8);
+            }
+        }
+        float u[2][4], z[4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) u[i][r] = (b2 ? v[i + 2][r] : v[i][r]) + __shfl_xor_sync(0xffffffffu, b2 ? v[i][r] : v[i + 2][r], 4);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) z[r] = (b1 ? u[1][r] : u[0][r]) + __shfl_xor_sync(0xffffffffu, b1 ? u[0][r] : u[1][r], 2);
+        const float w0 = (b0 ? z[2] : z[0]) + __shfl_xor_sync(0xffffffffu, b0 ? z[0] : z[2], 1);
+        const float w1 = (b0 ? z[3] : z[1]) + __shfl_xor_sync(0xffffffffu, b0 ? z[1] : z[3], 1);
+        const int row = 16 * warp + 8 * lr + (b3 ? 4 : 0) + (b2 ? 2 : 0) + (b1 ? 1 : 0), r0 = rb + (b0 ? 2 : 0);
+        X[r0 * 128 + row] = w0;
+        X[(r0 + 1) * 128 + row] = w1;
+    }
+}
+// Modified Gram-Schmidt of the R columns of X [R][128], warps 0 .. R - 1: warp j owns column j (lane = rows lane + 32 i) and takes
+// the earlier columns out of it in the order 0, 1, ....  A round makes TWO columns a, b final: the five sums |a|^2, a.b, |b|^2, a.x,
+// b.x (x: the warp's own column) come out of one reduction, and the products with b' = b - (q_a.b) q_a follow from them,
+//   |b'|^2 = |b|^2 - (q_a.b)^2,  b'.x' = b.x - (q_a.b) (q_a.x),
+// as long as b' keeps a quarter of |b|^2 -- then the differences cost two bits at most; where it does not, or where a sum left the
+// range of fp32, they are summed from the vectors themselves, the pairwise form.  R / 2 rounds, R products side by side, in
+// place of R (R + 1) / 2 reductions one after the other by one warp.  X is overwritten; on return x holds warp j's column.
+template <int R>
+__device__ __forceinline__ void qz_mgs(float* X, float (&x)[4], int warp, int lane) {
+    if (warp >= R) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = X[warp * 128 + lane + 32 * i];
+#pragma unroll 1
+    for (int c = 0; c < R; c += 2) {
+        float a[4], b[4], g[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            a[i] = X[c * 128 + lane + 32 * i];
+            b[i] = X[(c + 1) * 128 + lane + 32 * i];
+            g[0] = fmaf(a[i], a[i], g[0]); g[1] = fmaf(a[i], b[i], g[1]); g[2] = fmaf(b[i], b[i], g[2]);
+            g[3] = fmaf(a[i], x[i], g[3]); g[4] = fmaf(b[i], x[i], g[4]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < 5; ++k) g[k] += __shfl_xor_sync(0xffffffffu, g[k], o);
+        const bool in_range = fabsf(g[0]) + fabsf(g[1]) + fabsf(g[2]) + fabsf(g[3]) + fabsf(g[4]) <= 3.4e38f;
+        const float na = rsqrtf(fmaxf(g[0], 1e-30f));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] *= na;
+        float t = g[1] * na, s = g[3] * na;
+        if (!in_range) {                          // (the same in every lane) with the normalised column
+            t = s = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { t = fmaf(a[i], b[i], t); s = fmaf(a[i], x[i], s); }
+            t = warp_sum(t);
+            s = warp_sum(s);
+        }
+        float gb = fmaf(-t, t, g[2]), e = fmaf(-t, s, g[4]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) b[i] = fmaf(-t, a[i], b[i]);
+        if (warp > c)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = fmaf(-s, a[i], x[i]);
+        if (!in_range || !(gb >= 0.25f * g[2])) {
+            gb = e = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { gb = fmaf(b[i], b[i], gb); e = fmaf(b[i], x[i], e); }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) { gb += __shfl_xor_sync(0xffffffffu, gb, o); e += __shfl_xor_sync(0xffffffffu, e, o); }
+        }
+        const float nb = rsqrtf(fmaxf(gb, 1e-30f));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) b[i] *= nb;
+        if (warp == c) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = a[i];
+        } else if (warp == c + 1) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = b[i];
+        } else {
+            e *= nb;
+            if (!(fabsf(e) <= 3.4e38f)) {
+                e = 0.f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) e = fmaf(b[i], x[i], e);
+                e = warp_sum(e);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = fmaf(-e, b[i], x[i]);
+            if (warp < c + 4) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) X[warp * 128 + lane + 32 * i] = x[i];
+            }
+        }
+        if (warp < c + 2) return;                 // this warp's column is final
+        named_bar(1 + (c >> 1), 32 * (R - c - 2));
+    }
+}
+
+template <int R>
+__global__ void __launch_bounds__(NT_LA, 2)
 quantize_kernel(lq_dims d, char* __restrict__ ssm, float* __restrict__ Wbuf, float* __restrict__ Pbuf,
                 uint16_t* __restrict__ Gbuf, int32_t* __restrict__ hcnt, const float* __restrict__ Q0,
-                const int32_t* __restrict__ idx, int kda, int iters) {
-    extern __shared__ __align__(16) float smem[];
-    float* S = smem;                      // [128][LDB]
-    float* Qs = S + 128 * LDB;            // [128][R]
-    float* Ps = Qs + 128 * R;             // [128][R]
-    float* scr = Ps + 128 * R;            // [128][R]
-    float* sk = scr + 128 * R;            // [128]
-    float* part = sk + 128;               // [2][128]; afterwards [0 .. 127] holds 1 / Sk
-    const int tid = threadIdx.x;
-    const int n = blockIdx.x / d.HV, hv = blockIdx.x % d.HV;
-    const int slot = idx[n];
-    if (slot <= 0 || slot >= d.NS) return;
-    char* base = head_base(ssm, d.SS, slot, hv);
-
-    // the head's 64 KB arrive as 128 bulk asynchronous copies (one row of 512 bytes each, issued by 128 threads at once) that
-    // complete on one mbarrier: the whole tile is in flight from the first instruction on and costs no registers
+                const int32_t* __restrict__ idx, int nheads, int kda, int iters) {
+    extern __shared__ __align__(128) char qz_smem[];
+    float* tile = reinterpret_cast<float*>(qz_smem);                   // [128][128] the head to come
+    float* part = tile + 128 * 128;                                    // [8][R][128] partial products; also X = S P, |E| sums
+    float* X = part + 8 * R * 128;                                     // [R][128] P^T, later U^T
+    float2* Qd = reinterpret_cast<float2*>(X + R * 128);               // [128][R] Q, every value twice
+    float* Q0s = reinterpret_cast<float*>(Qd + 128 * R);               // [128][R] the start of the iteration
+    float* rsk = part + 8 * 128;                                       // [128] 1 / Sk (behind the sums of |E|, which part holds then)
+    float* rowf = rsk + 128;                                           // [128] 127 / Sv
     __shared__ __align__(8) uint64_t load_bar;
+    __shared__ int s_slot[2];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lc = lane & 15, lr = lane >> 4;
+    const int first = blockIdx.x, stride = gridDim.x;
+
+    auto slot_of = [&](int k) { const int p = first + k * stride; return p < nheads ? idx[p / d.HV] : 0; };
+    auto usable = [&](int slot) { return slot > 0 && slot < d.NS; };
+    auto fetch = [&](int k, int slot) {   // (thread 0)
+        mbar_arrive_expect_tx(&load_bar, uint32_t(QZ_TILE));
+        const char* src = head_base(ssm, d.SS, slot, (first + k * stride) % d.HV);
+        bulk_g2s(qz_smem, src, QZ_TILE, &load_bar);
+    };
     if (tid == 0) {
         mbar_init(&load_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_smem();
+        const int s0 = slot_of(0);
+        s_slot[0] = s0;
+        if (usable(s0)) fetch(0, s0);
     }
-    __syncthreads();
-    if (tid == 0) mbar_arrive_expect_tx(&load_bar, 128u * 512u);
-    __syncthreads();
-    if (tid < 128) bulk_g2s(S + tid * LDB, base + tid * 512, 512u, &load_bar);
-    for (int i = tid; i < 128 * R; i += NT_LA) Qs[i] = Q0[i];
-    {
-        bool ok = false;
-        for (uint32_t it = 0; it < WAIT_LIMIT && !ok; ++it) ok = mbar_try_wait(&load_bar, 0u);
-        if (!ok) atomicOr(&g_status, ST_FLUSH_TIMEOUT);
-    }
-    __syncthreads();
-
-    for (int it = 0; it < iters; ++it) {
-        coldot<R>(S, Qs, Ps, scr, tid);       // P = S^T Q
-        mgs_cols<R>(Ps, tid);
-        rowdot<R>(S, Ps, Qs, scr, tid);       // Q = S P
-        mgs_cols<R>(Qs, tid);
-    }
-    coldot<R>(S, Qs, Ps, scr, tid);           // U = S^T Q
-    for (int i = tid; i < 128 * R; i += NT_LA) {
-        Ps[i] = round_f16(Ps[i]);
-        Qs[i] = round_f16(Qs[i]);
-    }
-    __syncthreads();
-
-    // residual E = S - Q U^T (one factor at a time, fused multiply-add), column sums of |E|
-    {
-        const int c = tid & 127, half = tid >> 7;
-        float u[R];
+    for (int i = tid; i < R * 128; i += NT_LA) Q0s[i] = Q0[i];
+    uint32_t phase = 0;
+    for (int k = 0; first + k * stride < nheads; ++k) {
+        __syncthreads();                  // the slot of this head is known; everything of the head before is done
+        const int slot = s_slot[k & 1];
+        const bool on = usable(slot);
+        bool ok = true;
+        QzTile t;
+        if (on) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) u[r] = Ps[c * R + r];
-        float cs = 0.f;
-#pragma unroll 4
-        for (int row = half * 64; row < half * 64 + 64; ++row) {
-            float acc = S[row * LDB + c];
+            for (int u = 0; u < R / 2; ++u) {                          // Q <- Q0
+                const float q = Q0s[tid + u * NT_LA];
+                Qd[tid + u * NT_LA] = make_float2(q, q);
+            }
+            ok = warp_wait_bounded(&load_bar, phase, lane);
+            phase ^= 1u;
 #pragma unroll
-            for (int r = 0; r < R; ++r) acc = fmaf(-Qs[row * R + r], u[r], acc);
-            S[row * LDB + c] = acc;
-            cs += fabsf(acc);
+            for (int i = 0; i < 8; ++i) {
+                const float* row = tile + (16 * warp + 8 * lr + i) * 128 + 4 * lc;
+                const float4 lo = *reinterpret_cast<const float4*>(row), hi = *reinterpret_cast<const float4*>(row + 64);
+                t.s[i][0] = make_float2(lo.x, lo.y); t.s[i][1] = make_float2(lo.z, lo.w);
+                t.s[i][2] = make_float2(hi.x, hi.y); t.s[i][3] = make_float2(hi.z, hi.w);
+            }
         }
-        part[half * 128 + c] = cs;
-    }
-    __syncthreads();
-    if (tid < 128) {
-        const float skv = fmaxf(sqrtf((part[tid] + part[128 + tid]) / float(VD)), EPS);
-        sk[tid] = skv;
-        reinterpret_cast<float*>(base + CK_SK)[tid] = skv;
-        part[tid] = 1.0f / skv;               // (its own partial sums were read just above)
-    }
-    __syncthreads();
-    quant_rows_div(S, sk, part, base, tid);
+        if (!__syncthreads_and(ok)) {     // the tile never came: nothing is written, the status word says why
+            if (tid == 0) atomicOr(&g_status, ST_FLUSH_TIMEOUT);
+            return;
+        }
+        // The tile is in registers and the next head's may come.  (It is only ever read through the generic proxy, and those reads
+        // are behind the barrier: no proxy fence, which would also wait for the thread's stores to the head before.)
+        auto fetch_next = [&] {           // (one thread)
+            const int nx = slot_of(k + 1);
+            s_slot[(k + 1) & 1] = nx;
+            if (usable(nx)) fetch(k + 1, nx);
+        };
+        if (!on) {
+            if (tid == 0) fetch_next();
+            continue;
+        }
+        const int hv = (first + k * stride) % d.HV;
+        char* base = head_base(ssm, d.SS, slot, hv);
+        const int64_t sh = int64_t(slot) * d.HV + hv;
 
-    uint16_t* uq = reinterpret_cast<uint16_t*>(base + CK_UQ);
-    for (int i = tid; i < R * 128; i += NT_LA) {
-        const int r = i >> 7, c = i & 127;
-        uq[r * (KD + VD) + c] = f_to_f16(Ps[c * R + r]);
-        uq[r * (KD + VD) + KD + c] = f_to_f16(Qs[c * R + r]);
+        // Work that does not wait for the arithmetic, done by four warps that have nothing to do in the first Gram-Schmidt (R = 4:
+        // the warps without a column; R = 8: those whose columns are final first): the next head's copy, the window reset.
+        auto aside = [&] {
+            const int at = R == 4 ? tid - 128 : tid;
+            if (at < 0 || at >= 128) return;
+            if (at == 0) fetch_next();
+            for (int j = at; j < d.L; j += 128) Wbuf[sh * d.L + j] = 0.f;
+            if (kda) {
+                Pbuf[sh * KD + at] = 0.f;
+                uint4* g4 = reinterpret_cast<uint4*>(Gbuf + sh * d.L * KD);
+                for (int i = at; i < d.L * KD / 8; i += 128) g4[i] = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);     // fp16 1.0
+            } else if (at == 1) {
+                Pbuf[sh] = 1.f;
+            }
+            if (at == 1) hcnt[sh] = 0;
+        };
+        // half steps: P = S^T Q, orthonormalised; Q = S P, orthonormalised; ...; U = S^T Q (one copy of each piece of code: a head
+        // runs through this loop body once from a cold instruction cache)
+#pragma unroll 1
+        for (int hs = 0;; ++hs) {
+            const bool to_q = hs & 1, last = hs >= 2 * iters;
+            if (to_q) {
+                qz_rowdot<R>(t, X, part, warp, lane);
+            } else {
+                qz_coldot<R>(t, Qd, part, warp, lane);
+                __syncthreads();
+                qz_sum_parts<R>(part, X, tid, last);
+                if (last) {
+                    if (hs == 0) aside();
+                    break;
+                }
+            }
+            __syncthreads();
+            float x[4];
+            qz_mgs<R>(to_q ? part : X, x, warp, lane);
+            if (hs == 0) aside();
+            if (!to_q) __syncthreads();   // (the raw columns are read until the last round is over)
+            if (warp < R) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (to_q) Qd[(lane + 32 * i) * R + warp] = make_float2(x[i], x[i]);
+                    else X[warp * 128 + lane + 32 * i] = x[i];
+                }
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+
+        // residual E = S - Q U^T in place (one factor at a time, fused multiply-add), column sums of |E|
+#pragma unroll 1
+        for (int rb = 0; rb < R; rb += 4) {
+            float2 u[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float4 lo = *reinterpret_cast<const float4*>(X + (rb + r) * 128 + 4 * lc), hi = *reinterpret_cast<const float4*>(X + (rb + r) * 128 + 64 + 4 * lc);
+                u[r][0] = make_float2(lo.x, lo.y); u[r][1] = make_float2(lo.z, lo.w);
+                u[r][2] = make_float2(hi.x, hi.y); u[r][3] = make_float2(hi.z, hi.w);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float2* qrow = Qd + (16 * warp + 8 * lr + i) * R + rb;
+                const float4 qa = *reinterpret_cast<const float4*>(qrow), qb = *reinterpret_cast<const float4*>(qrow + 2);
+                // (both factors as they are stored: U was rounded to f16 as it was summed)
+                const float qv[4] = {-round_f16(qa.x), -round_f16(qa.z), -round_f16(qb.x), -round_f16(qb.z)};
+                const float2 q[4] = {make_float2(qv[0], qv[0]), make_float2(qv[1], qv[1]), make_float2(qv[2], qv[2]), make_float2(qv[3], qv[3])};
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) t.s[i][p] = __ffma2_rn(q[r], u[r][p], t.s[i][p]);
+            }
+        }
+        {
+            float cs[8];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                cs[2 * p] = fabsf(t.s[0][p].x); cs[2 * p + 1] = fabsf(t.s[0][p].y);
+#pragma unroll
+                for (int i = 1; i < 8; ++i) { cs[2 * p] += fabsf(t.s[i][p].x); cs[2 * p + 1] += fabsf(t.s[i][p].y); }
+            }
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = (lr ? cs[4 + j] : cs[j]) + __shfl_xor_sync(0xffffffffu, lr ? cs[j] : cs[4 + j], 16);
+            *reinterpret_cast<float4*>(part + warp * 128 + 64 * lr + 4 * lc) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+        __syncthreads();
+        if (tid < 128) {
+            float cs = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) cs += part[w * 128 + tid];
+            const float skv = fmaxf(sqrtf(cs / float(VD)), EPS);
+            rsk[tid] = 1.0f / skv;
+            reinterpret_cast<float*>(base + CK_SK)[tid] = skv;
+        }
+        {                                 // the factors, two values per word: a row is 64 words of U^T and 64 of Q^T
+            uint32_t* uq = reinterpret_cast<uint32_t*>(base + CK_UQ);
+#pragma unroll
+            for (int u = 0; u < R / 4; ++u) {
+                const int r = (tid >> 6) + 4 * u, e = tid & 63;
+                const __half2 hu = __floats2half2_rn(X[r * 128 + 2 * e], X[r * 128 + 2 * e + 1]);
+                const __half2 hq = __floats2half2_rn(Qd[2 * e * R + r].x, Qd[(2 * e + 1) * R + r].x);
+                uq[r * 128 + e] = *reinterpret_cast<const uint32_t*>(&hu);
+                uq[r * 128 + 64 + e] = *reinterpret_cast<const uint32_t*>(&hq);
+            }
+        }
+        __syncthreads();
+
+        // Row scales and codes: Sv[v] = max(max_c |E| (1 / Sk), EPS), code = rint(E (1 / Sk) (127 / Sv)), which is the reference's
+        // rint(E / (Sk Sv) * 127) (leapquant/kernels.py:2218-2229) wherever that lies further than 1e-4 code units from a rounding
+        // boundary: either form carries at most four fp32 roundings of a value of at most 127.  |E (1 / Sk)| <= Sv, so the clamp
+        // to +-127 never acts.  The sum with 1.5 * 2^23 rounds, and its low mantissa byte is the code in two's complement.
+        float rm[8];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const float2 k2 = *reinterpret_cast<const float2*>(rsk + (p >> 1) * 64 + 4 * lc + 2 * (p & 1));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                t.s[i][p] = __fmul2_rn(t.s[i][p], k2);
+                const float m = fmaxf(fabsf(t.s[i][p].x), fabsf(t.s[i][p].y));
+                rm[i] = p == 0 ? m : fmaxf(rm[i], m);
+            }
+        }
+        // the row maximum over sixteen lanes: lane bits 3..1 pick the row, bit 0 is folded last
+        const bool b3 = lc & 8, b2 = lc & 4, b1 = lc & 2;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rm[i] = fmaxf(b3 ? rm[i + 4] : rm[i], __shfl_xor_sync(0xffffffffu, b3 ? rm[i] : rm[i + 4], 8));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) rm[i] = fmaxf(b2 ? rm[i + 2] : rm[i], __shfl_xor_sync(0xffffffffu, b2 ? rm[i] : rm[i + 2], 4));
+        rm[0] = fmaxf(b1 ? rm[1] : rm[0], __shfl_xor_sync(0xffffffffu, b1 ? rm[0] : rm[1], 2));
+        rm[0] = fmaxf(rm[0], __shfl_xor_sync(0xffffffffu, rm[0], 1));
+        {
+            const int row = 16 * warp + 8 * lr + (lc >> 1);
+            const float svv = fmaxf(rm[0], EPS);
+            if (!(lc & 1)) {
+                reinterpret_cast<float*>(base + CK_SV)[row] = svv;
+                rowf[row] = QMAX / svv;
+            }
+        }
+        __syncwarp();
+        uint32_t* codes = reinterpret_cast<uint32_t*>(base + CK_CODES) + (16 * warp + 8 * lr) * 32 + lc;
+        const float2 mg = make_float2(RNE_MAGIC, RNE_MAGIC);
+        const float* rf = rowf + 16 * warp + 8 * lr;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float rv = rf[i];
+            const float2 rv2 = make_float2(rv, rv);
+            float2 z[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) z[p] = __ffma2_rn(t.s[i][p], rv2, mg);
+            codes[i * 32] = pack4(__float_as_uint(z[0].x), __float_as_uint(z[0].y), __float_as_uint(z[1].x), __float_as_uint(z[1].y));
+            codes[i * 32 + 16] = pack4(__float_as_uint(z[2].x), __float_as_uint(z[2].y), __float_as_uint(z[3].x), __float_as_uint(z[3].y));
+        }
+
     }
-    // window reset
-    const int64_t sh = int64_t(slot) * d.HV + hv;
-    for (int j = tid; j < d.L; j += NT_LA) Wbuf[sh * d.L + j] = 0.f;
-    if (kda) {
-        for (int c = tid; c < KD; c += NT_LA) Pbuf[sh * KD + c] = 0.f;
-        uint32_t* g32 = reinterpret_cast<uint32_t*>(Gbuf + sh * d.L * KD);
-        for (int i = tid; i < d.L * KD / 2; i += NT_LA) g32[i] = 0x3C003C00u;     // fp16 1.0 pairs
-    } else if (tid == 0) {
-        Pbuf[sh] = 1.f;
-    }
-    if (tid == 0) hcnt[sh] = 0;
 }
 
 // four 8 x 8 b16 tiles, transposed: lane l supplies the address of row l % 8 of tile l / 8 and receives, of each tile, the
@@ -573,15 +840,15 @@ extern "C" int lq_quantize(const lq_dims* d, void* ssm, float* Wbuf, float* Pbuf
     if (N < 0 || iters < 0) return LQ_ERR_RANGE;
     if (misaligned16({ssm}) || (kda && misaligned16({Gbuf}))) return LQ_ERR_ALIGN;
     if (N == 0) return LQ_OK;
-    const size_t smem = sizeof(float) * (128 * LDB + 3 * 128 * d->R + 128 + 256);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    dim3 grid(unsigned(N) * d->HV), block(NT_LA);
+    const int nheads = N * d->HV, cap = 2 * device_sm_count();
+    dim3 grid(unsigned(nheads < cap ? nheads : cap)), block(NT_LA);
     if (d->R == 4) {
-        if ((rc = ensure_smem((const void*)quantize_kernel<4>, smem))) return rc;
-        quantize_kernel<4><<<grid, block, smem, st>>>(*d, (char*)ssm, Wbuf, Pbuf, (uint16_t*)Gbuf, hcnt, Q0, idx, kda, iters);
+        if ((rc = ensure_smem((const void*)quantize_kernel<4>, qz_smem_bytes<4>()))) return rc;
+        quantize_kernel<4><<<grid, block, qz_smem_bytes<4>(), st>>>(*d, (char*)ssm, Wbuf, Pbuf, (uint16_t*)Gbuf, hcnt, Q0, idx, nheads, kda, iters);
     } else {
-        if ((rc = ensure_smem((const void*)quantize_kernel<8>, smem))) return rc;
-        quantize_kernel<8><<<grid, block, smem, st>>>(*d, (char*)ssm, Wbuf, Pbuf, (uint16_t*)Gbuf, hcnt, Q0, idx, kda, iters);
+        if ((rc = ensure_smem((const void*)quantize_kernel<8>, qz_smem_bytes<8>()))) return rc;
+        quantize_kernel<8><<<grid, block, qz_smem_bytes<8>(), st>>>(*d, (char*)ssm, Wbuf, Pbuf, (uint16_t*)Gbuf, hcnt, Q0, idx, nheads, kda, iters);
     }
     return finish_launch();
 }
