@@ -109,30 +109,35 @@ def conv1d(x, conv_state, weight, bias):
 def ptr(t):
     """Device address of a CUDA tensor's first element; refuses host tensors (no CPU path exists)."""
     if not t.is_cuda:
-        raise LeapQuantError("leapquant_b200 kernels take CUDA tensors only (there is no CPU fallback)")
+        not_cuda()
     return t.data_ptr()
 
 
+# torch's current stream of a device as a raw handle, and the current device, without the Python objects around them
+raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+current_device = torch._C._cuda_getDevice if hasattr(torch._C, "_cuda_getDevice") else torch.cuda.current_device
+
+
 def stream_of(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return raw_stream(t.get_device())
 
 
-class on_device:
-    """Makes the tensor's device current for the duration of a launch when it is not already."""
+def not_cuda():
+    raise LeapQuantError("leapquant_b200 kernels take CUDA tensors only (there is no CPU fallback)")
 
-    def __init__(self, t):
-        self.idx = t.device.index
-        self.prev = None
 
-    def __enter__(self):
-        cur = torch.cuda.current_device()
-        if cur != self.idx:
-            self.prev = cur
-            torch.cuda.set_device(self.idx)
-
-    def __exit__(self, *exc):
-        if self.prev is not None:
-            torch.cuda.set_device(self.prev)
+def launch(fn, what, t, *args):
+    """fn(*args, stream) on the device of the CUDA tensor `t`, made current for the call when it is not, and on torch's current
+    stream of that device; raises on an error code."""
+    dev = t.get_device()
+    if current_device() == dev:
+        rc = fn(*args, raw_stream(dev))
+    else:
+        with torch.cuda.device(dev):
+            rc = fn(*args, raw_stream(dev))
+    if rc != 0:
+        check(rc, what)
 
 
 def set_option(name, value):

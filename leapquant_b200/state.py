@@ -126,21 +126,28 @@ class LeapQuantState:
 
         mixed bf16 [N, 2HK + HV*V]; a: GDN (N, HV) | KDA (N, HV, K) raw gate; b (N, HV); dt_bias: GDN (HV,) | KDA (HV*K,);
         idx int (N,); out bf16 (N, HV, V) written in place.  No host synchronisation, no allocation when the dtypes match."""
-        A_log = A_log if A_log.dtype == torch.float32 else self._p32(A_log)
-        dt_bias = dt_bias if dt_bias.dtype == torch.float32 else self._p32(dt_bias)
-        KA = self.K if self.kda else 1
-        a = a.reshape(a.shape[0], self.HV, KA).contiguous()
-        dt_bias = dt_bias.reshape(self.HV, KA).contiguous()
-        idx = idx if idx.dtype == torch.int32 else idx.to(torch.int32)
-        v = self.views(ssm)
+        if A_log.dtype != torch.float32:
+            A_log = self._p32(A_log)
+        if dt_bias.dtype != torch.float32:
+            dt_bias = self._p32(dt_bias)
+        # the kernels take addresses: a tensor that is contiguous and has the right number of elements is passed as it is
+        HV, KA = self.HV, self.K if self.kda else 1
+        if not a.is_contiguous() or a.numel() != a.shape[0] * HV * KA:
+            a = a.reshape(a.shape[0], HV, KA).contiguous()
+        if not dt_bias.is_contiguous() or dt_bias.numel() != HV * KA:
+            dt_bias = dt_bias.reshape(HV, KA).contiguous()
+        if idx.dtype != torch.int32:
+            idx = idx.to(torch.int32)
         if self.fused:
+            q = ssm if ssm.dim() == 4 else self.views(ssm)["q32"]         # (the checkpoint begins where the fp32 slot does)
             if self.kda:
-                self.kdecode(v["q32"], self.Kbuf, self.Ubuf, self.Wbuf, self.Pbuf, self.Gbuf, self.hcnt, mixed, a, b, A_log,
+                self.kdecode(q, self.Kbuf, self.Ubuf, self.Wbuf, self.Pbuf, self.Gbuf, self.hcnt, mixed, a, b, A_log,
                              dt_bias, self.Q0, idx, out, self.work)
             else:
-                self.kdecode(v["q32"], self.Kbuf, self.Ubuf, self.Wbuf, self.Pbuf, self.hcnt, mixed, a, b, A_log, dt_bias,
+                self.kdecode(q, self.Kbuf, self.Ubuf, self.Wbuf, self.Pbuf, self.hcnt, mixed, a, b, A_log, dt_bias,
                              self.Q0, idx, out, self.work)
             return
+        v = self.views(ssm)
         if self.kda:
             self.kstep(v["q32"], v["Sk"], v["Sv"], v["skv"], self.Kbuf, self.Ubuf, self.Wbuf, self.Pbuf, self.Gbuf,
                        self.hcnt, mixed, a, b, A_log, dt_bias, v["uq"], idx, out)
@@ -165,7 +172,7 @@ class LeapQuantState:
                 self._kconv = KN.make_conv1d_update(self.NS, C)
             if self._mixed is None or self._mixed.shape[0] < N:
                 self._mixed = torch.empty(max(N, 64), C, dtype=torch.bfloat16, device=x.device)
-            mixed = self._mixed[:N]
+            mixed = self._mixed if self._mixed.shape[0] == N else self._mixed[:N]
             i32 = idx if idx.dtype == torch.int32 else idx.to(torch.int32)
             self._kconv(x, conv_state, conv_weight, conv_bias, i32, mixed)
             return self.decode(ssm, mixed, a, b, A_log, dt_bias, i32, out)
