@@ -161,12 +161,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // A whole warp waits for the phase with the given parity: lane 0 tests the barrier, the outcome is broadcast, and every
 // lane takes the same branch, so the warp stays converged (a lane that spins alone leaves the warp split in two, and every
 // later warp-synchronous shuffle then costs a rendezvous of the halves).  Gives up after WAIT_LIMIT polls.
+// Only lane 0 has acquired the phase's data by then, and a shuffle orders no memory: the __syncwarp puts what the other lanes
+// read next behind lane 0's acquire.
 __device__ __forceinline__ bool warp_wait_bounded(uint64_t* bar, uint32_t parity, int lane) {
     for (uint32_t it = 0; it < WAIT_LIMIT; ++it) {
         uint32_t ok = 0;
         if (lane == 0) ok = mbar_try_wait(bar, parity) ? 1u : 0u;
         ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (ok) return true;
+        if (ok) {
+            __syncwarp();
+            return true;
+        }
     }
     return false;
 }
