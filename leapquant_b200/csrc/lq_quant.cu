@@ -253,7 +253,7 @@ quantize_kernel(lq_dims d, char* __restrict__ ssm, float* __restrict__ Wbuf, flo
                 const float q = Q0s[tid + u * NT_LA];
                 Qd[tid + u * NT_LA] = make_float2(q, q);
             }
-            ok = warp_wait_bounded(&load_bar, phase, lane);
+            ok = warp_wait_bounded(&load_bar, phase);
             phase ^= 1u;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -532,7 +532,7 @@ dequant_kernel(lq_dims d, char* __restrict__ ssm, const uint16_t* __restrict__ K
                 }
             }
             const int s = i & 1;
-            if (i >= 2 && !warp_wait_bounded(empty + s, uint32_t((i >> 1) - 1) & 1u, lane)) {
+            if (i >= 2 && !warp_wait_bounded(empty + s, uint32_t((i >> 1) - 1) & 1u)) {
                 if (lane == 0) atomicOr(&g_status, ST_PRODUCER_TIMEOUT);
                 return;
             }
@@ -571,7 +571,7 @@ dequant_kernel(lq_dims d, char* __restrict__ ssm, const uint16_t* __restrict__ K
     for (int i = 0; first + i * stride < nheads; ++i) {
     const int s = i & 1;
     if (warp == 0) {
-        const bool got = warp_wait_bounded(full + s, uint32_t(i >> 1) & 1u, lane);
+        const bool got = warp_wait_bounded(full + s, uint32_t(i >> 1) & 1u);
         if (lane == 0) *okflag = got ? 1 : 0;
     }
     named_bar(1, NT_LA);                                  // (also: every warp is done with the previous head's operands and window rows)

@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(UT + NG * GT, 1) step_pipelined_kernel(StepPar
                 while (tail < i) {                               // reclaim in order until the stage and its descriptor are free
                     const uint32_t vt = __shfl_sync(0xffffffffu, r_vs, tail % ND);
                     if (v1 - vt <= uint32_t(ring_bytes) && i - tail < ND) break;
-                    if (!warp_wait_bounded(empty + (tail % ND), uint32_t(tail / ND) & 1u, lane)) { ok = false; break; }
+                    if (!warp_wait_bounded(empty + (tail % ND), uint32_t(tail / ND) & 1u)) { ok = false; break; }
                     ++tail;
                 }
                 if (!ok) {
@@ -980,7 +980,7 @@ __global__ void __launch_bounds__(UT + NG * GT, 1) step_pipelined_kernel(StepPar
         const uint64_t keep_policy = l2_policy_evict_last();
         for (int i = 0; i < nit; ++i) {
             const int dsc = i % ND;
-            if (!warp_wait_bounded(ready + dsc, uint32_t(i / ND) & 1u, lane)) {
+            if (!warp_wait_bounded(ready + dsc, uint32_t(i / ND) & 1u)) {
                 if (lane == 0) { atomicOr(&g_status, ST_PRODUCER_TIMEOUT); *abortf = 1; }
                 return;
             }
@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(UT + NG * GT, 1) step_pipelined_kernel(StepPar
         // one program of this warp ahead: row and key head follow from the program index alone
         auto run_prologue = [&](int i, const uint2& q_cur, const uint2& k_cur) -> bool {
             const int dsc = i % ND;
-            if (!warp_wait_bounded(full + dsc, uint32_t(i / ND) & 1u, lane)) {
+            if (!warp_wait_bounded(full + dsc, uint32_t(i / ND) & 1u)) {
                 if (lane == 0) { atomicOr(&g_status, ST_PROLOGUE_TIMEOUT); *abortf = 1; }
                 return false;
             }
@@ -1135,7 +1135,7 @@ __global__ void __launch_bounds__(UT + NG * GT, 1) step_pipelined_kernel(StepPar
         const int dsc = i % ND;
         // one warp polls and publishes the outcome; the other warps sleep at the group barrier
         if (t < 32) {
-            const bool got = warp_wait_bounded(normed + dsc, uint32_t(i / ND) & 1u, t);
+            const bool got = warp_wait_bounded(normed + dsc, uint32_t(i / ND) & 1u);
             if (t == 0) *gflag = got ? 1 : 0;
         }
         named_bar(bar, GT);

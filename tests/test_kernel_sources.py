@@ -2,8 +2,6 @@
 import os
 import re
 
-import pytest
-
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "leapquant_b200", "csrc")
 
 
@@ -18,17 +16,16 @@ def body(text, name):
             return text[at:i + 1]
 
 
-@pytest.mark.parametrize("name", ["warp_wait_bounded"])
-def test_broadcast_wait_orders_the_warp(name):
-    """One lane tests the barrier and a shuffle tells the others, which orders no memory: before the function reports success the
-    warp has to synchronise, or the other lanes may read shared memory from before the copy they waited for."""
-    b = body(open(os.path.join(CSRC, "lq_common.cuh")).read(), name)
-    poll, told, sync, done = (b.index(s) for s in ("mbar_try_wait(", "__shfl_sync(", "__syncwarp()", "return true"))
-    assert poll < told < sync < done
+def test_every_lane_acquires():
+    """A wait of a warp: a lane that learns of the phase from another (a shuffle, a vote) has acquired nothing and may read shared
+    memory from before the copy it waited for, so every lane has to have tested the barrier itself."""
+    b = body(open(os.path.join(CSRC, "lq_common.cuh")).read(), "warp_wait_bounded")
+    assert "if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;" in b
+    assert "lane" not in b and "shfl" not in b
 
 
-def test_one_lane_waits_only_through_it():
-    """Every other wait on a barrier is one that each thread makes for itself."""
+def test_no_lane_waits_alone():
+    """Nor does any other wait on a barrier hang on one lane."""
     for f in sorted(os.listdir(CSRC)):
         if f.endswith((".cu", ".cuh")):
             text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, f)).read())
