@@ -1,8 +1,8 @@
 // Standalone quantize, in-place dequantize and low-rank factorisation kernels (sm_100a).
 //
-// Quantize: persistent CTAs, a head's 128 x 128 fp32 tile in the registers of one CTA, the next head's on its way into shared
-// memory.  Dequantize: persistent CTAs that walk the heads, each head's checkpoint staged in shared memory.  Low-rank: one CTA
-// of 256 threads per matrix, which stays in shared memory.
+// Quantize: persistent CTAs, a head's 128 x 128 fp32 tile in shared memory and its residual in the registers of one CTA.
+// Dequantize: persistent CTAs that walk the heads, each head's checkpoint staged in shared memory.  Low-rank: one CTA of 256
+// threads per matrix, which stays in shared memory.
 // Either way the in-place rewrite of a slot (fp32 state <-> packed 8-bit checkpoint) never reads what it has already
 // overwritten.
 #include "lq_linalg.cuh"
@@ -12,376 +12,306 @@ namespace lq {
 // ------------------------------------------------------------------------------------------------------------------
 // quantize
 // ------------------------------------------------------------------------------------------------------------------
-// One head = one 128 x 128 fp32 tile, held in REGISTERS by the 256 threads of a CTA (64 values each) from the moment it has
-// arrived until its codes are stored; persistent CTAs, two per SM.  The tile is read from shared memory once, so that the
-// buffer is free for the next head's 64 KB -- one bulk asynchronous copy, in flight during the whole of this head's
-// arithmetic -- and every product of the subspace iteration works on registers with packed f32x2 multiply-adds (two fp32
-// products per instruction, each rounded as the scalar one would be).
-// Thread (warp w, lane): lc = lane % 16, lr = lane / 16 owns rows 16 w + 8 lr + i (i < 8) and columns 4 lc .. + 3, 64 + 4 lc .. + 3.
-//   P = S^T Q: 8 rows are summed in the thread, two half-warps by one exchange, eight warps through shared memory.
-//   Q = S P:   8 columns in the thread, sixteen lanes by halving exchanges; a warp ends with its own 16 rows.
-// What bounds it: issue slots of the sixteen resident warps (R = 4: 14 400 warp instructions per head, a third of them the
-// multiply-adds, issued in 39 % of the cycles); the previous form read the tile from shared memory for every product (32 000
-// instructions per head, three CTAs per SM).  Dequantize + quantize of 8 192 GDN heads: 496 -> 390 us, of 416 heads 39 -> 36 us,
-// of 1 536 KDA heads (R = 8, three iterations) 277 -> 214 us.
-constexpr int QZ_TILE = 128 * 128 * 4;
+// One head = one 128 x 128 fp32 tile in shared memory; persistent CTAs of 128 threads, three per SM.
+// Requantizing a state is discontinuous (a rounding of one pass is a code of the next), so every sum here has ONE order, that of
+// lq_lowrank's products: 64 + 64 terms in index order, the two halves added last; Gram-Schmidt pair by pair in the order of the
+// columns.  What that leaves to choose is how many sums a thread carries side by side:
+//   P = S^T Q: a thread has C columns and four factors; a half-warp sums the first 64 rows, the other the second.
+//   Q = S P:   the same with C rows.
+//   Residual and column sums of |E|: as P, two columns with their factors in registers.
+//   Row scales and codes: eight lanes share a row, a warp has 32 rows.
+// Shared memory delivers 128 bytes a cycle, broadcasts included, and C columns with four factors take 4 / C + 1 bytes per
+// multiply-add: 2 560 cycles per product of four factors with C = 1, which was the bound of the form before (a row or a column per
+// thread, 256 threads), 1 536 with C = 2, 1 024 with C = 4.  R = 4: C = 2 keeps all four warps busy (C = 4 on half of them:
+// 459 us where C = 2 takes 430).  R = 8: C = 4, a pair of warps per four factors.
+// The tile is eight pieces of sixteen rows, 16 bytes apart, one bulk asynchronous copy each (a copy per row holds the issuing warp
+// up for 8 000 cycles): eight lanes that take the same columns of eight rows hit different banks if the rows are of eight pieces.
+// What is left is latency: a head is a chain of ten phases between barriers for twelve warps per SM.  Dequantize + quantize against
+// a row or a column per thread (same sums): 8 192 GDN heads 495 -> 368 us, 416 heads 38.4 -> 31.7 us, 1 536 KDA heads 278 -> 191 us.
+constexpr int QZ_THREADS = 128, QZ_CTAS = 3;
+constexpr int QZ_PIECE = 16 * 128 + 4;                                  // floats
+__device__ __forceinline__ constexpr int qz_at(int row) { return (row >> 4) * QZ_PIECE + (row & 15) * 128; }
 template <int R>
-__host__ __device__ constexpr int qz_smem_bytes() { return QZ_TILE + 8 * R * 128 * 4 + R * 128 * 4 + R * 128 * 8 + R * 128 * 4; }
+__host__ __device__ constexpr int qz_smem_bytes() { return 8 * QZ_PIECE * 4 + (R == 4 ? 3 : 2) * R * 128 * 4 + 2 * 128 * 4 + 16; }
 
-struct QzTile {
-    float2 s[8][4];                       // [row i][column pair]: pairs 0, 1 = columns 4 lc .. + 3; 2, 3 = 64 + 4 lc .. + 3
-};
-// partial products over the warp's 16 rows: part[w][r][c] = sum_row S[row][c] Q[row][r]; Qd: [128][R] values duplicated to pairs
-template <int R>
-__device__ __forceinline__ void qz_coldot(const QzTile& t, const float2* __restrict__ Qd, float* __restrict__ part, int warp, int lane) {
-    const int lc = lane & 15, lr = lane >> 4;
-    const float2* qrow = Qd + (16 * warp + 8 * lr) * R;
-    float* out = part + warp * (R * 128) + 64 * lr + 4 * lc;
-#pragma unroll 1
-    for (int rb = 0; rb < R; rb += 4) {
-        float2 acc[4][4];                 // [column pair][r]
+// a[.] += m x for four factors x
+__device__ __forceinline__ void qz_fma(float (&a)[4], float m, const float4& x) {
+    a[0] = fmaf(m, x.x, a[0]);
+    a[1] = fmaf(m, x.y, a[1]);
+    a[2] = fmaf(m, x.z, a[2]);
+    a[3] = fmaf(m, x.w, a[3]);
+}
+// v + the other half-warp's v
+__device__ __forceinline__ float qz_halves(float v) { return v + __shfl_xor_sync(0xffffffffu, v, 16); }
+// The half-warps' sums of C outputs (at `step` floats from each other) times four factors are added and stored, half of them by
+// each half-warp; on request rounded to f16 values.
+template <int C>
+__device__ __forceinline__ void qz_put(float* __restrict__ Y, int step, const float (&acc)[C][4], int half, bool round16) {
+    float4 v[C];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float4 qa = *reinterpret_cast<const float4*>(qrow + i * R + rb), qb = *reinterpret_cast<const float4*>(qrow + i * R + rb + 2);
-            const float2 q[4] = {make_float2(qa.x, qa.y), make_float2(qa.z, qa.w), make_float2(qb.x, qb.y), make_float2(qb.z, qb.w)};
+    for (int i = 0; i < C; ++i) v[i] = make_float4(qz_halves(acc[i][0]), qz_halves(acc[i][1]), qz_halves(acc[i][2]), qz_halves(acc[i][3]));
 #pragma unroll
-            for (int p = 0; p < 4; ++p)
-#pragma unroll
-                for (int r = 0; r < 4; ++r) acc[p][r] = i == 0 ? __fmul2_rn(t.s[i][p], q[r]) : __ffma2_rn(t.s[i][p], q[r], acc[p][r]);
-        }
-        // the half-warp lr keeps the columns 64 lr + 4 lc .. + 3
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            float v[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float2 lo = acc[k >> 1][r], hi = acc[2 + (k >> 1)][r];
-                const float a = (k & 1) ? lo.y : lo.x, b = (k & 1) ? hi.y : hi.x;
-                v[k] = (lr ? b : a) + __shfl_xor_sync(0xffffffffu, lr ? a : b, 16);
-            }
-            *reinterpret_cast<float4*>(out + (rb + r) * 128) = make_float4(v[0], v[1], v[2], v[3]);
-        }
+    for (int i = 0; i < C / 2; ++i) {
+        float4 w = half ? v[C / 2 + i] : v[i];
+        if (round16) w = make_float4(round_f16(w.x), round_f16(w.y), round_f16(w.z), round_f16(w.w));
+        *reinterpret_cast<float4*>(Y + (C / 2 * half + i) * step) = w;
     }
 }
-// X[r][c] = sum over the eight warps' partials (all 256 threads), on request rounded to f16 values
-template <int R>
-__device__ __forceinline__ void qz_sum_parts(const float* __restrict__ part, float* __restrict__ X, int tid, bool round16) {
-    constexpr int PT = R * 128 / NT_LA;   // outputs per thread: 2 or 4
-    float a[PT];
-#pragma unroll
-    for (int k = 0; k < PT; ++k) a[k] = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-        if constexpr (PT == 2) {
-            const float2 v = *reinterpret_cast<const float2*>(part + w * (R * 128) + 2 * tid);
-            a[0] += v.x; a[1] += v.y;
-        } else {
-            const float4 v = *reinterpret_cast<const float4*>(part + w * (R * 128) + 4 * tid);
-            a[0] += v.x; a[1] += v.y; a[2] += v.z; a[3] += v.w;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < PT; ++k) X[PT * tid + k] = round16 ? round_f16(a[k]) : a[k];
-}
-// X[r][row] = sum_c S[row][c] P[r][c]
-template <int R>
-__device__ __forceinline__ void qz_rowdot(const QzTile& t, const float* __restrict__ P, float* __restrict__ X, int warp, int lane) {
-    const int lc = lane & 15, lr = lane >> 4;
-    const bool b3 = lc & 8, b2 = lc & 4, b1 = lc & 2, b0 = lc & 1;
-#pragma unroll 1
-    for (int rb = 0; rb < R; rb += 4) {
-        float v[4][4];                    // [row i or i + 4, by bit 3 of lc][r]
-        float2 pv[4][4];                  // [r][column pair]
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const float4 lo = *reinterpret_cast<const float4*>(P + (rb + r) * 128 + 4 * lc), hi = *reinterpret_cast<const float4*>(P + (rb + r) * 128 + 64 + 4 * lc);
-            pv[r][0] = make_float2(lo.x, lo.y); pv[r][1] = make_float2(lo.z, lo.w);
-            pv[r][2] = make_float2(hi.x, hi.y); pv[r][3] = make_float2(hi.z, hi.w);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                float2 x = __fmul2_rn(t.s[i][0], pv[r][0]), y = __fmul2_rn(t.s[i + 4][0], pv[r][0]);
-#pragma unroll
-                for (int p = 1; p < 4; ++p) {
-                    x = __ffma2_rn(t.s[i][p], pv[r][p], x);
-                    y = __ffma2_rn(t.s[i + 4][p], pv[r][p], y);
-                }
-                const float xs = x.x + x.y, ys = y.x + y.y;
-                v[i][r] = (b3 ? ys : xs) + __shfl_xor_sync(0xffffffffu, b3 ? xs : ys, 8);
-            }
-        }
-        float u[2][4], z[4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) u[i][r] = (b2 ? v[i + 2][r] : v[i][r]) + __shfl_xor_sync(0xffffffffu, b2 ? v[i][r] : v[i + 2][r], 4);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) z[r] = (b1 ? u[1][r] : u[0][r]) + __shfl_xor_sync(0xffffffffu, b1 ? u[0][r] : u[1][r], 2);
-        const float w0 = (b0 ? z[2] : z[0]) + __shfl_xor_sync(0xffffffffu, b0 ? z[0] : z[2], 1);
-        const float w1 = (b0 ? z[3] : z[1]) + __shfl_xor_sync(0xffffffffu, b0 ? z[1] : z[3], 1);
-        const int row = 16 * warp + 8 * lr + (b3 ? 4 : 0) + (b2 ? 2 : 0) + (b1 ? 1 : 0), r0 = rb + (b0 ? 2 : 0);
-        X[r0 * 128 + row] = w0;
-        X[(r0 + 1) * 128 + row] = w1;
+// C consecutive floats
+template <int C>
+__device__ __forceinline__ void qz_get(float (&v)[C], const float* __restrict__ p) {
+    if constexpr (C == 2) {
+        const float2 x = *reinterpret_cast<const float2*>(p);
+        v[0] = x.x; v[1] = x.y;
+    } else {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
     }
 }
-// Modified Gram-Schmidt of the R columns of X [R][128], warps 0 .. R - 1: warp j owns column j (lane = rows lane + 32 i) and takes
-// the earlier columns out of it in the order 0, 1, ....  A round makes TWO columns a, b final: the five sums |a|^2, a.b, |b|^2, a.x,
-// b.x (x: the warp's own column) come out of one reduction, and the products with b' = b - (q_a.b) q_a follow from them,
-//   |b'|^2 = |b|^2 - (q_a.b)^2,  b'.x' = b.x - (q_a.b) (q_a.x),
-// as long as b' keeps a quarter of |b|^2 -- then the differences cost two bits at most; where it does not, or where a sum left the
-// range of fp32, they are summed from the vectors themselves, the pairwise form.  R / 2 rounds, R products side by side, in
-// place of R (R + 1) / 2 reductions one after the other by one warp.  X is overwritten; on return x holds warp j's column.
+// Modified Gram-Schmidt of the R columns of X [128][R] by one warp (lane = rows lane + 32 i).  As soon as a column is final it is
+// taken out of all later ones: each of these still loses the columns 0, 1, ... in that order, as in mgs_cols, but a column costs
+// two reductions one after the other and not one per pair.
 template <int R>
-__device__ __forceinline__ void qz_mgs(float* X, float (&x)[4], int warp, int lane) {
-    if (warp >= R) return;
+__device__ __forceinline__ void qz_mgs(float* __restrict__ X, int lane) {
+    float x[4][R];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = X[warp * 128 + lane + 32 * i];
-#pragma unroll 1
-    for (int c = 0; c < R; c += 2) {
-        float a[4], b[4], g[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            a[i] = X[c * 128 + lane + 32 * i];
-            b[i] = X[(c + 1) * 128 + lane + 32 * i];
-            g[0] = fmaf(a[i], a[i], g[0]); g[1] = fmaf(a[i], b[i], g[1]); g[2] = fmaf(b[i], b[i], g[2]);
-            g[3] = fmaf(a[i], x[i], g[3]); g[4] = fmaf(b[i], x[i], g[4]);
+        for (int r = 0; r < R; r += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(X + (lane + 32 * i) * R + r);
+            x[i][r] = a.x; x[i][r + 1] = a.y; x[i][r + 2] = a.z; x[i][r + 3] = a.w;
+        }
+#pragma unroll
+    for (int c = 0; c < R; ++c) {
+        float n = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) n = fmaf(x[i][c], x[i][c], n);
+        n = rsqrtf(fmaxf(warp_sum(n), 1e-30f));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i][c] *= n;
+        float s[R];
+#pragma unroll
+        for (int j = c + 1; j < R; ++j) {
+            s[j] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[j] = fmaf(x[i][c], x[i][j], s[j]);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-            for (int k = 0; k < 5; ++k) g[k] += __shfl_xor_sync(0xffffffffu, g[k], o);
-        const bool in_range = fabsf(g[0]) + fabsf(g[1]) + fabsf(g[2]) + fabsf(g[3]) + fabsf(g[4]) <= 3.4e38f;
-        const float na = rsqrtf(fmaxf(g[0], 1e-30f));
+            for (int j = c + 1; j < R; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] *= na;
-        float t = g[1] * na, s = g[3] * na;
-        if (!in_range) {                          // (the same in every lane) with the normalised column
-            t = s = 0.f;
+        for (int j = c + 1; j < R; ++j)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { t = fmaf(a[i], b[i], t); s = fmaf(a[i], x[i], s); }
-            t = warp_sum(t);
-            s = warp_sum(s);
-        }
-        float gb = fmaf(-t, t, g[2]), e = fmaf(-t, s, g[4]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) b[i] = fmaf(-t, a[i], b[i]);
-        if (warp > c)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = fmaf(-s, a[i], x[i]);
-        if (!in_range || !(gb >= 0.25f * g[2])) {
-            gb = e = 0.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { gb = fmaf(b[i], b[i], gb); e = fmaf(b[i], x[i], e); }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) { gb += __shfl_xor_sync(0xffffffffu, gb, o); e += __shfl_xor_sync(0xffffffffu, e, o); }
-        }
-        const float nb = rsqrtf(fmaxf(gb, 1e-30f));
-#pragma unroll
-        for (int i = 0; i < 4; ++i) b[i] *= nb;
-        if (warp == c) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = a[i];
-        } else if (warp == c + 1) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = b[i];
-        } else {
-            e *= nb;
-            if (!(fabsf(e) <= 3.4e38f)) {
-                e = 0.f;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) e = fmaf(b[i], x[i], e);
-                e = warp_sum(e);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = fmaf(-e, b[i], x[i]);
-            if (warp < c + 4) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) X[warp * 128 + lane + 32 * i] = x[i];
-            }
-        }
-        if (warp < c + 2) return;                 // this warp's column is final
-        named_bar(1 + (c >> 1), 32 * (R - c - 2));
+            for (int i = 0; i < 4; ++i) x[i][j] = fmaf(-s[j], x[i][c], x[i][j]);
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int r = 0; r < R; r += 4) *reinterpret_cast<float4*>(X + (lane + 32 * i) * R + r) = make_float4(x[i][r], x[i][r + 1], x[i][r + 2], x[i][r + 3]);
 }
 
 template <int R>
-__global__ void __launch_bounds__(NT_LA, 2)
+__global__ void __launch_bounds__(QZ_THREADS, QZ_CTAS)
 quantize_kernel(lq_dims d, char* __restrict__ ssm, float* __restrict__ Wbuf, float* __restrict__ Pbuf,
                 uint16_t* __restrict__ Gbuf, int32_t* __restrict__ hcnt, const float* __restrict__ Q0,
                 const int32_t* __restrict__ idx, int nheads, int kda, int iters) {
     extern __shared__ __align__(128) char qz_smem[];
-    float* tile = reinterpret_cast<float*>(qz_smem);                   // [128][128] the head to come
-    float* part = tile + 128 * 128;                                    // [8][R][128] partial products; also X = S P, |E| sums
-    float* X = part + 8 * R * 128;                                     // [R][128] P^T, later U^T
-    float2* Qd = reinterpret_cast<float2*>(X + R * 128);               // [128][R] Q, every value twice
-    float* Q0s = reinterpret_cast<float*>(Qd + 128 * R);               // [128][R] the start of the iteration
-    float* rsk = part + 8 * 128;                                       // [128] 1 / Sk (behind the sums of |E|, which part holds then)
-    float* rowf = rsk + 128;                                           // [128] 127 / Sv
-    __shared__ __align__(8) uint64_t load_bar;
-    __shared__ int s_slot[2];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lc = lane & 15, lr = lane >> 4;
+    float* S = reinterpret_cast<float*>(qz_smem);                      // the state, later the residual, then the head to come
+    float* Ps = S + 8 * QZ_PIECE;                                      // [128][R] P, at the end U as it is stored
+    float* Qs = Ps + 128 * R;                                          // [128][R] Q
+    float* Qh = R == 4 ? Qs + 128 * R : Qs;                            // [128][R] -Q as it is stored
+    float* sk = Qh + 128 * R;                                          // [128] Sk
+    float* rsk = sk + 128;                                             // [128] 1 / Sk
+    uint64_t* load_bar = reinterpret_cast<uint64_t*>(rsk + 128);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int l16 = lane & 15, half = lane >> 4;                        // sums: a half-warp has one half of the terms
     const int first = blockIdx.x, stride = gridDim.x;
 
     auto slot_of = [&](int k) { const int p = first + k * stride; return p < nheads ? idx[p / d.HV] : 0; };
     auto usable = [&](int slot) { return slot > 0 && slot < d.NS; };
-    auto fetch = [&](int k, int slot) {   // (thread 0)
-        mbar_arrive_expect_tx(&load_bar, uint32_t(QZ_TILE));
-        const char* src = head_base(ssm, d.SS, slot, (first + k * stride) % d.HV);
-        bulk_g2s(qz_smem, src, QZ_TILE, &load_bar);
+    auto fetch = [&](int k, int slot, int p) {      // piece p of the k-th head (one thread; eight arrivals complete the phase)
+        mbar_arrive_expect_tx(load_bar, 8192u);
+        bulk_g2s(S + p * QZ_PIECE, head_base(ssm, d.SS, slot, (first + k * stride) % d.HV) + p * 8192, 8192u, load_bar);
     };
     if (tid == 0) {
-        mbar_init(&load_bar, 1);
+        mbar_init(load_bar, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
-        const int s0 = slot_of(0);
-        s_slot[0] = s0;
-        if (usable(s0)) fetch(0, s0);
     }
-    for (int i = tid; i < R * 128; i += NT_LA) Q0s[i] = Q0[i];
+    int slot = slot_of(0);
+    __syncthreads();
+    if (lane < 2 && usable(slot)) fetch(0, slot, 2 * warp + lane);
     uint32_t phase = 0;
     for (int k = 0; first + k * stride < nheads; ++k) {
-        __syncthreads();                  // the slot of this head is known; everything of the head before is done
-        const int slot = s_slot[k & 1];
-        const bool on = usable(slot);
-        bool ok = true;
-        QzTile t;
-        if (on) {
-#pragma unroll
-            for (int u = 0; u < R / 2; ++u) {                          // Q <- Q0
-                const float q = Q0s[tid + u * NT_LA];
-                Qd[tid + u * NT_LA] = make_float2(q, q);
-            }
-            ok = warp_wait_bounded(&load_bar, phase);
-            phase ^= 1u;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float* row = tile + (16 * warp + 8 * lr + i) * 128 + 4 * lc;
-                const float4 lo = *reinterpret_cast<const float4*>(row), hi = *reinterpret_cast<const float4*>(row + 64);
-                t.s[i][0] = make_float2(lo.x, lo.y); t.s[i][1] = make_float2(lo.z, lo.w);
-                t.s[i][2] = make_float2(hi.x, hi.y); t.s[i][3] = make_float2(hi.z, hi.w);
-            }
+        const int next = slot_of(k + 1);
+        if (!usable(slot)) {
+            if (lane < 2 && usable(next)) fetch(k + 1, next, 2 * warp + lane);      // (its own pieces: it has read the last of them)
+            slot = next;
+            continue;
         }
+#pragma unroll
+        for (int u = 0; u < R / 4; ++u) {                              // Q <- Q0
+            const int e = 4 * (tid + u * QZ_THREADS);
+            *reinterpret_cast<float4*>(Qs + e) = make_float4(Q0[e], Q0[e + 1], Q0[e + 2], Q0[e + 3]);
+        }
+        bool ok = warp_wait_bounded(load_bar, phase);
+        if (!ok) ok = warp_wait_bounded(load_bar, phase);              // (nobody leaves while a copy into its memory is on its way)
+        phase ^= 1u;
         if (!__syncthreads_and(ok)) {     // the tile never came: nothing is written, the status word says why
             if (tid == 0) atomicOr(&g_status, ST_FLUSH_TIMEOUT);
             return;
-        }
-        // The tile is in registers and the next head's may come.  (It is only ever read through the generic proxy, and those reads
-        // are behind the barrier: no proxy fence, which would also wait for the thread's stores to the head before.)
-        auto fetch_next = [&] {           // (one thread)
-            const int nx = slot_of(k + 1);
-            s_slot[(k + 1) & 1] = nx;
-            if (usable(nx)) fetch(k + 1, nx);
-        };
-        if (!on) {
-            if (tid == 0) fetch_next();
-            continue;
         }
         const int hv = (first + k * stride) % d.HV;
         char* base = head_base(ssm, d.SS, slot, hv);
         const int64_t sh = int64_t(slot) * d.HV + hv;
 
-        // Work that does not wait for the arithmetic, done by four warps that have nothing to do in the first Gram-Schmidt (R = 4:
-        // the warps without a column; R = 8: those whose columns are final first): the next head's copy, the window reset.
-        auto aside = [&] {
-            const int at = R == 4 ? tid - 128 : tid;
-            if (at < 0 || at >= 128) return;
-            if (at == 0) fetch_next();
-            for (int j = at; j < d.L; j += 128) Wbuf[sh * d.L + j] = 0.f;
-            if (kda) {
-                Pbuf[sh * KD + at] = 0.f;
-                uint4* g4 = reinterpret_cast<uint4*>(Gbuf + sh * d.L * KD);
-                for (int i = at; i < d.L * KD / 8; i += 128) g4[i] = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);     // fp16 1.0
-            } else if (at == 1) {
-                Pbuf[sh] = 1.f;
+        auto round_q = [&] {
+            for (int e = 4 * tid; e < R * 128; e += 4 * QZ_THREADS) {
+                const float4 q = *reinterpret_cast<const float4*>(Qs + e);
+                *reinterpret_cast<float4*>(Qh + e) = make_float4(-round_f16(q.x), -round_f16(q.y), -round_f16(q.z), -round_f16(q.w));
             }
-            if (at == 1) hcnt[sh] = 0;
         };
         // half steps: P = S^T Q, orthonormalised; Q = S P, orthonormalised; ...; U = S^T Q (one copy of each piece of code: a head
         // runs through this loop body once from a cold instruction cache)
 #pragma unroll 1
         for (int hs = 0;; ++hs) {
             const bool to_q = hs & 1, last = hs >= 2 * iters;
-            if (to_q) {
-                qz_rowdot<R>(t, X, part, warp, lane);
-            } else {
-                qz_coldot<R>(t, Qd, part, warp, lane);
-                __syncthreads();
-                qz_sum_parts<R>(part, X, tid, last);
-                if (last) {
-                    if (hs == 0) aside();
-                    break;
-                }
-            }
-            __syncthreads();
-            float x[4];
-            qz_mgs<R>(to_q ? part : X, x, warp, lane);
-            if (hs == 0) aside();
-            if (!to_q) __syncthreads();   // (the raw columns are read until the last round is over)
-            if (warp < R) {
+            if (R == 4 && last) round_q();
+            // R = 4: two rows or columns per thread; R = 8: four, and a pair of warps per four factors
+            constexpr int C = R / 2;
+            {
+                const int r0 = R == 8 ? 4 * (warp >> 1) : 0, w = R == 8 ? warp & 1 : warp;
+                float acc[C][4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (to_q) Qd[(lane + 32 * i) * R + warp] = make_float2(x[i], x[i]);
-                    else X[warp * 128 + lane + 32 * i] = x[i];
-                }
-            }
-            __syncthreads();
-        }
-        __syncthreads();
-
-        // residual E = S - Q U^T in place (one factor at a time, fused multiply-add), column sums of |E|
+                for (int i = 0; i < C; ++i)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) acc[i][r] = 0.f;
+                const float* x = (to_q ? Ps : Qs) + 64 * half * R + r0;
+                // rows of Q = S P: 16 (l16 % 8) + 2 C w + l16 / 8 + 2 i, eight lanes of eight pieces; columns of P = S^T Q: C side by side
+                const int at = to_q ? 16 * (l16 & 7) + 2 * C * w + (l16 >> 3) : C * (16 * w + l16);
+                if (to_q) {
+                    const float* m = S + qz_at(at) + 64 * half;
+#pragma unroll 4
+                    for (int c = 0; c < 64; c += 4) {
+                        float4 mv[C], xv[4];
+#pragma unroll
+                        for (int i = 0; i < C; ++i) mv[i] = *reinterpret_cast<const float4*>(m + 2 * i * 128 + c);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) xv[i] = *reinterpret_cast<const float4*>(x + (c + i) * R);
+#pragma unroll
+                        for (int i = 0; i < C; ++i) qz_fma(acc[i], mv[i].x, xv[0]);
+#pragma unroll
+                        for (int i = 0; i < C; ++i) qz_fma(acc[i], mv[i].y, xv[1]);
+#pragma unroll
+                        for (int i = 0; i < C; ++i) qz_fma(acc[i], mv[i].z, xv[2]);
+#pragma unroll
+                        for (int i = 0; i < C; ++i) qz_fma(acc[i], mv[i].w, xv[3]);
+                    }
+                } else {
+                    const float* m = S + 4 * half * QZ_PIECE + at;
 #pragma unroll 1
-        for (int rb = 0; rb < R; rb += 4) {
-            float2 u[4][4];
+                    for (int p = 0; p < 4; ++p, m += QZ_PIECE, x += 16 * R)
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float4 lo = *reinterpret_cast<const float4*>(X + (rb + r) * 128 + 4 * lc), hi = *reinterpret_cast<const float4*>(X + (rb + r) * 128 + 64 + 4 * lc);
-                u[r][0] = make_float2(lo.x, lo.y); u[r][1] = make_float2(lo.z, lo.w);
-                u[r][2] = make_float2(hi.x, hi.y); u[r][3] = make_float2(hi.z, hi.w);
+                        for (int row = 0; row < 16; ++row) {
+                            float mv[C];
+                            qz_get<C>(mv, m + row * 128);
+                            const float4 xv = *reinterpret_cast<const float4*>(x + row * R);
+#pragma unroll
+                            for (int i = 0; i < C; ++i) qz_fma(acc[i], mv[i], xv);
+                        }
+                }
+                qz_put<C>((to_q ? Qs : Ps) + at * R + r0, to_q ? 2 * R : R, acc, half, last);
             }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float2* qrow = Qd + (16 * warp + 8 * lr + i) * R + rb;
-                const float4 qa = *reinterpret_cast<const float4*>(qrow), qb = *reinterpret_cast<const float4*>(qrow + 2);
-                // (both factors as they are stored: U was rounded to f16 as it was summed)
-                const float qv[4] = {-round_f16(qa.x), -round_f16(qa.z), -round_f16(qb.x), -round_f16(qb.z)};
-                const float2 q[4] = {make_float2(qv[0], qv[0]), make_float2(qv[1], qv[1]), make_float2(qv[2], qv[2]), make_float2(qv[3], qv[3])};
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) t.s[i][p] = __ffma2_rn(q[r], u[r][p], t.s[i][p]);
+            __syncthreads();
+            const int mw = (first + hs) & 3;                           // the warp that orthonormalises
+            if (hs == 0 && warp != mw) {
+                // work that does not wait for the arithmetic, by the other three: the window reset
+                const int at = ((warp - mw - 1) & 3) * 32 + lane;
+#pragma unroll 1
+                for (int j = at; j < d.L; j += 96) Wbuf[sh * d.L + j] = 0.f;
+                if (kda) {
+                    for (int c = at; c < KD; c += 96) Pbuf[sh * KD + c] = 0.f;
+                    uint4* g4 = reinterpret_cast<uint4*>(Gbuf + sh * d.L * KD);
+#pragma unroll 2
+                    for (int i = at; i < d.L * KD / 8; i += 96) g4[i] = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);     // fp16 1.0
+                } else if (at == 1) {
+                    Pbuf[sh] = 1.f;
+                }
+                if (at == 1) hcnt[sh] = 0;
             }
+            if (last) break;
+            if (warp == mw) qz_mgs<R>(to_q ? Qs : Ps, lane);
+            __syncthreads();
         }
+        if (R == 8) {                                                  // (in place: the products are through with Q)
+            round_q();
+            __syncthreads();
+        }
+
         {
-            float cs[8];
+            // residual E = S - Q U^T over the state (one factor at a time, fused multiply-add), column sums of |E|, column scales
+            const int col = 2 * (16 * warp + l16);                     // of this thread: col, col + 1
+            float4 u[2][R / 4];
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                cs[2 * p] = fabsf(t.s[0][p].x); cs[2 * p + 1] = fabsf(t.s[0][p].y);
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int i = 1; i < 8; ++i) { cs[2 * p] += fabsf(t.s[i][p].x); cs[2 * p + 1] += fabsf(t.s[i][p].y); }
+                for (int r = 0; r < R / 4; ++r) u[i][r] = *reinterpret_cast<const float4*>(Ps + (col + i) * R + 4 * r);
+            float* m = S + 4 * half * QZ_PIECE + col;
+            const float* x = Qh + 64 * half * R;
+            float cs[2] = {0.f, 0.f};
+            constexpr int NB = 4;                                      // rows in a batch: loaded before those of the batch before are stored
+            float2 mv[NB];
+            float4 xv[NB][R / 4];
+            auto load = [&](int row) {
+#pragma unroll
+                for (int i = 0; i < NB; ++i) {
+                    mv[i] = *reinterpret_cast<const float2*>(m + qz_at(row) + i * 128);
+#pragma unroll
+                    for (int r = 0; r < R / 4; ++r) xv[i][r] = *reinterpret_cast<const float4*>(x + (row + i) * R + 4 * r);
+                }
+            };
+            load(0);
+#pragma unroll 2
+            for (int row = 0; row < 64; row += NB) {
+                float e[NB][2];
+#pragma unroll
+                for (int i = 0; i < NB; ++i) {
+                    e[i][0] = mv[i].x; e[i][1] = mv[i].y;
+#pragma unroll
+                    for (int r = 0; r < R / 4; ++r) {
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) e[i][c] = fmaf(xv[i][r].x, u[c][r].x, e[i][c]);
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) e[i][c] = fmaf(xv[i][r].y, u[c][r].y, e[i][c]);
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) e[i][c] = fmaf(xv[i][r].z, u[c][r].z, e[i][c]);
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) e[i][c] = fmaf(xv[i][r].w, u[c][r].w, e[i][c]);
+                    }
+                }
+                load(row + NB < 64 ? row + NB : 0);                    // (the last is not used)
+#pragma unroll
+                for (int i = 0; i < NB; ++i) {
+                    cs[0] += fabsf(e[i][0]);
+                    cs[1] += fabsf(e[i][1]);
+                    *reinterpret_cast<float2*>(m + qz_at(row) + i * 128) = make_float2(e[i][0], e[i][1]);
+                }
             }
-            float v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = (lr ? cs[4 + j] : cs[j]) + __shfl_xor_sync(0xffffffffu, lr ? cs[j] : cs[4 + j], 16);
-            *reinterpret_cast<float4*>(part + warp * 128 + 64 * lr + 4 * lc) = make_float4(v[0], v[1], v[2], v[3]);
-        }
-        __syncthreads();
-        if (tid < 128) {
-            float cs = 0.f;
-#pragma unroll
-            for (int w = 0; w < 8; ++w) cs += part[w * 128 + tid];
-            const float skv = fmaxf(sqrtf(cs / float(VD)), EPS);
-            rsk[tid] = 1.0f / skv;
-            reinterpret_cast<float*>(base + CK_SK)[tid] = skv;
-        }
-        {                                 // the factors, two values per word: a row is 64 words of U^T and 64 of Q^T
+            fence_async_smem();           // these stores come before the copy of the next head
+            cs[0] = qz_halves(cs[0]);
+            cs[1] = qz_halves(cs[1]);
+            const float skv = fmaxf(sqrtf((half ? cs[1] : cs[0]) / float(VD)), EPS);
+            sk[col + half] = skv;
+            rsk[col + half] = 1.0f / skv;
+            reinterpret_cast<float*>(base + CK_SK)[col + half] = skv;
+            // the factors, two values per word: a row is 64 words of U^T and 64 of Q^T
             uint32_t* uq = reinterpret_cast<uint32_t*>(base + CK_UQ);
-#pragma unroll
-            for (int u = 0; u < R / 4; ++u) {
-                const int r = (tid >> 6) + 4 * u, e = tid & 63;
-                const __half2 hu = __floats2half2_rn(X[r * 128 + 2 * e], X[r * 128 + 2 * e + 1]);
-                const __half2 hq = __floats2half2_rn(Qd[2 * e * R + r].x, Qd[(2 * e + 1) * R + r].x);
+            const int e = tid & 63;
+#pragma unroll 2
+            for (int r = tid >> 6; r < R; r += 2) {
+                const __half2 hu = __floats2half2_rn(Ps[2 * e * R + r], Ps[(2 * e + 1) * R + r]);
+                const __half2 hq = __floats2half2_rn(-Qh[2 * e * R + r], -Qh[(2 * e + 1) * R + r]);
                 uq[r * 128 + e] = *reinterpret_cast<const uint32_t*>(&hu);
                 uq[r * 128 + 64 + e] = *reinterpret_cast<const uint32_t*>(&hq);
             }
@@ -391,49 +321,58 @@ quantize_kernel(lq_dims d, char* __restrict__ ssm, float* __restrict__ Wbuf, flo
         // Row scales and codes: Sv[v] = max(max_c |E| (1 / Sk), EPS), code = rint(E (1 / Sk) (127 / Sv)), which is the reference's
         // rint(E / (Sk Sv) * 127) (leapquant/kernels.py:2218-2229) wherever that lies further than 1e-4 code units from a rounding
         // boundary: either form carries at most four fp32 roundings of a value of at most 127.  |E (1 / Sk)| <= Sv, so the clamp
-        // to +-127 never acts.  The sum with 1.5 * 2^23 rounds, and its low mantissa byte is the code in two's complement.
-        float rm[8];
+        // to +-127 never acts.
+        // A warp has two pieces of the tile, a lane four rows of each; the next head's copy of a piece is started as soon as the warp
+        // is through with it.
+        const int l8 = lane & 7;
+        float2 rk[8];                                                  // of columns 4 l8 + 32 j .. + 3, j < 4
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const float2 k2 = *reinterpret_cast<const float2*>(rsk + (p >> 1) * 64 + 4 * lc + 2 * (p & 1));
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(rsk + 4 * l8 + 32 * j);
+            rk[2 * j] = make_float2(v.x, v.y);
+            rk[2 * j + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll 1
+        for (int it = 0; it < 2; ++it) {
+            const int row0 = 32 * warp + 16 * it + (lane >> 3);        // rows row0 + 4 i, i < 4: of one piece
+            const float* E = S + qz_at(row0);
+            float2 a[4][8];                                            // E (1 / Sk)
+            float best[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                t.s[i][p] = __fmul2_rn(t.s[i][p], k2);
-                const float m = fmaxf(fabsf(t.s[i][p].x), fabsf(t.s[i][p].y));
-                rm[i] = p == 0 ? m : fmaxf(rm[i], m);
+            for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 v = *reinterpret_cast<const float4*>(E + 4 * i * 128 + 4 * l8 + 32 * j);
+                    a[i][2 * j] = __fmul2_rn(make_float2(v.x, v.y), rk[2 * j]);
+                    a[i][2 * j + 1] = __fmul2_rn(make_float2(v.z, v.w), rk[2 * j + 1]);
+                    const float m = fmaxf(fmaxf(fabsf(a[i][2 * j].x), fabsf(a[i][2 * j].y)), fmaxf(fabsf(a[i][2 * j + 1].x), fabsf(a[i][2 * j + 1].y)));
+                    best[i] = j == 0 ? m : fmaxf(best[i], m);
+                }
             }
-        }
-        // the row maximum over sixteen lanes: lane bits 3..1 pick the row, bit 0 is folded last
-        const bool b3 = lc & 8, b2 = lc & 4, b1 = lc & 2;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) rm[i] = fmaxf(b3 ? rm[i + 4] : rm[i], __shfl_xor_sync(0xffffffffu, b3 ? rm[i] : rm[i + 4], 8));
+            for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) rm[i] = fmaxf(b2 ? rm[i + 2] : rm[i], __shfl_xor_sync(0xffffffffu, b2 ? rm[i] : rm[i + 2], 4));
-        rm[0] = fmaxf(b1 ? rm[1] : rm[0], __shfl_xor_sync(0xffffffffu, b1 ? rm[0] : rm[1], 2));
-        rm[0] = fmaxf(rm[0], __shfl_xor_sync(0xffffffffu, rm[0], 1));
-        {
-            const int row = 16 * warp + 8 * lr + (lc >> 1);
-            const float svv = fmaxf(rm[0], EPS);
-            if (!(lc & 1)) {
-                reinterpret_cast<float*>(base + CK_SV)[row] = svv;
-                rowf[row] = QMAX / svv;
+                for (int i = 0; i < 4; ++i) best[i] = fmaxf(best[i], __shfl_xor_sync(0xffffffffu, best[i], o));
+            const float2 mg = make_float2(RNE_MAGIC, RNE_MAGIC);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                best[i] = fmaxf(best[i], EPS);
+                const float rv = QMAX / best[i];
+                if (l8 == 0) reinterpret_cast<float*>(base + CK_SV)[row0 + 4 * i] = best[i];
+                uint32_t* codes = reinterpret_cast<uint32_t*>(base + CK_CODES) + (row0 + 4 * i) * 32 + l8;
+                const float2 rv2 = make_float2(rv, rv);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    // rint() by adding 1.5 * 2^23: the sum's low mantissa byte is the code in two's complement
+                    const float2 x = a[i][2 * j], y = a[i][2 * j + 1];
+                    const float2 tx = __ffma2_rn(x, rv2, mg), ty = __ffma2_rn(y, rv2, mg);
+                    codes[8 * j] = pack4(__float_as_uint(tx.x), __float_as_uint(tx.y), __float_as_uint(ty.x), __float_as_uint(ty.y));
+                }
             }
+            __syncwarp();                                              // every lane has read the last of the piece
+            if (lane == 0 && usable(next)) fetch(k + 1, next, 2 * warp + it);
         }
-        __syncwarp();
-        uint32_t* codes = reinterpret_cast<uint32_t*>(base + CK_CODES) + (16 * warp + 8 * lr) * 32 + lc;
-        const float2 mg = make_float2(RNE_MAGIC, RNE_MAGIC);
-        const float* rf = rowf + 16 * warp + 8 * lr;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float rv = rf[i];
-            const float2 rv2 = make_float2(rv, rv);
-            float2 z[4];
-#pragma unroll
-            for (int p = 0; p < 4; ++p) z[p] = __ffma2_rn(t.s[i][p], rv2, mg);
-            codes[i * 32] = pack4(__float_as_uint(z[0].x), __float_as_uint(z[0].y), __float_as_uint(z[1].x), __float_as_uint(z[1].y));
-            codes[i * 32 + 16] = pack4(__float_as_uint(z[2].x), __float_as_uint(z[2].y), __float_as_uint(z[3].x), __float_as_uint(z[3].y));
-        }
-
+        slot = next;
     }
 }
 
@@ -841,8 +780,8 @@ extern "C" int lq_quantize(const lq_dims* d, void* ssm, float* Wbuf, float* Pbuf
     if (misaligned16({ssm}) || (kda && misaligned16({Gbuf}))) return LQ_ERR_ALIGN;
     if (N == 0) return LQ_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int nheads = N * d->HV, cap = 2 * device_sm_count();
-    dim3 grid(unsigned(nheads < cap ? nheads : cap)), block(NT_LA);
+    const int nheads = N * d->HV, cap = QZ_CTAS * device_sm_count();
+    dim3 grid(unsigned(nheads < cap ? nheads : cap)), block(QZ_THREADS);
     if (d->R == 4) {
         if ((rc = ensure_smem((const void*)quantize_kernel<4>, qz_smem_bytes<4>()))) return rc;
         quantize_kernel<4><<<grid, block, qz_smem_bytes<4>(), st>>>(*d, (char*)ssm, Wbuf, Pbuf, (uint16_t*)Gbuf, hcnt, Q0, idx, nheads, kda, iters);
