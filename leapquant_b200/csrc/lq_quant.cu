@@ -26,11 +26,14 @@ namespace lq {
 // 459 us where C = 2 takes 430).  R = 8: C = 4, a pair of warps per four factors.
 // The tile is eight pieces of sixteen rows, 16 bytes apart, one bulk asynchronous copy each (a copy per row holds the issuing warp
 // up for 8 000 cycles): eight lanes that take the same columns of eight rows hit different banks if the rows are of eight pieces.
-// What is left is latency: a head is a chain of ten phases between barriers for twelve warps per SM.  Dequantize + quantize against
-// a row or a column per thread (same sums): 8 192 GDN heads 495 -> 368 us, 416 heads 38.4 -> 31.7 us, 1 536 KDA heads 278 -> 191 us.
+// What is left is latency: a head is a chain of ten phases between barriers for twelve warps per SM.  R = 4: 20 000 warp instructions
+// per head, issued in 49 % of the cycles; R = 8, three iterations: 53 500 in 42 %, a third of the stalls at barriers while one warp
+// orthonormalises.  Dequantize + quantize against a row or a column per thread (same bits): 8 192 GDN heads 495 -> 421 us, 416
+// heads 39.4 -> 36.1 us, 1 536 KDA heads 278 -> 203 us.
 constexpr int QZ_THREADS = 128, QZ_CTAS = 3;
 constexpr int QZ_PIECE = 16 * 128 + 4;                                  // floats
 __device__ __forceinline__ constexpr int qz_at(int row) { return (row >> 4) * QZ_PIECE + (row & 15) * 128; }
+constexpr float TIE_BAND = 6e-5f;                                       // code units, see below
 template <int R>
 __host__ __device__ constexpr int qz_smem_bytes() { return 8 * QZ_PIECE * 4 + (R == 4 ? 3 : 2) * R * 128 * 4 + 2 * 128 * 4 + 16; }
 
@@ -318,10 +321,13 @@ quantize_kernel(lq_dims d, char* __restrict__ ssm, float* __restrict__ Wbuf, flo
         }
         __syncthreads();
 
-        // Row scales and codes: Sv[v] = max(max_c |E| (1 / Sk), EPS), code = rint(E (1 / Sk) (127 / Sv)), which is the reference's
-        // rint(E / (Sk Sv) * 127) (leapquant/kernels.py:2218-2229) wherever that lies further than 1e-4 code units from a rounding
-        // boundary: either form carries at most four fp32 roundings of a value of at most 127.  |E (1 / Sk)| <= Sv, so the clamp
-        // to +-127 never acts.
+        // Row scales and codes are those of the reference's true divisions (leapquant/kernels.py:2218-2229),
+        //   Sv[v] = max(max_c |E / Sk|, EPS),  code = clamp(rint(E / (Sk Sv) * 127)),
+        // but a division is only executed where it can matter.  Row maximum: the candidates are found with |E| (1 / Sk) (within two
+        // ulp of the quotient), and only elements within 1e-6 of the best candidate are divided -- the true maximum is always among
+        // them.  Codes: y = E (1 / Sk) (127 / Sv) and the reference's expression carry six fp32 roundings of a value of at most
+        // 127 between them, 4.6e-5, so rint(y) is the code unless y lies within TIE_BAND of a half-integer, and only then is the
+        // expression evaluated.  |y| <= 127 (1 + 3e-7) by construction of Sv: the clamp never acts.
         // A warp has two pieces of the tile, a lane four rows of each; the next head's copy of a piece is started as soon as the warp
         // is through with it.
         const int l8 = lane & 7;
@@ -337,7 +343,7 @@ quantize_kernel(lq_dims d, char* __restrict__ ssm, float* __restrict__ Wbuf, flo
             const int row0 = 32 * warp + 16 * it + (lane >> 3);        // rows row0 + 4 i, i < 4: of one piece
             const float* E = S + qz_at(row0);
             float2 a[4][8];                                            // E (1 / Sk)
-            float best[4];
+            float cm[4][4], thr[4], best[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
 #pragma unroll
@@ -345,15 +351,45 @@ quantize_kernel(lq_dims d, char* __restrict__ ssm, float* __restrict__ Wbuf, flo
                     const float4 v = *reinterpret_cast<const float4*>(E + 4 * i * 128 + 4 * l8 + 32 * j);
                     a[i][2 * j] = __fmul2_rn(make_float2(v.x, v.y), rk[2 * j]);
                     a[i][2 * j + 1] = __fmul2_rn(make_float2(v.z, v.w), rk[2 * j + 1]);
-                    const float m = fmaxf(fmaxf(fabsf(a[i][2 * j].x), fabsf(a[i][2 * j].y)), fmaxf(fabsf(a[i][2 * j + 1].x), fabsf(a[i][2 * j + 1].y)));
-                    best[i] = j == 0 ? m : fmaxf(best[i], m);
+                    cm[i][j] = fmaxf(fmaxf(fabsf(a[i][2 * j].x), fabsf(a[i][2 * j].y)), fmaxf(fabsf(a[i][2 * j + 1].x), fabsf(a[i][2 * j + 1].y)));
                 }
+                thr[i] = fmaxf(fmaxf(fmaxf(cm[i][0], cm[i][1]), fmaxf(cm[i][2], cm[i][3])), 0.f);
             }
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
+                for (int i = 0; i < 4; ++i) thr[i] = fmaxf(thr[i], __shfl_xor_sync(0xffffffffu, thr[i], o));
+            uint32_t hit = 0;                                          // four columns of a row with a candidate among them
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                thr[i] *= 1.0f - 1e-6f;
+                best[i] = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) hit |= cm[i][j] >= thr[i] ? 1u << (4 * i + j) : 0u;
+            }
+            while (hit) {
+                const int at = __ffs(hit) - 1, i = at >> 2, c0 = 4 * l8 + 32 * (at & 3);
+                hit &= hit - 1;
+                const float4 e = *reinterpret_cast<const float4*>(E + 4 * i * 128 + c0), q = *reinterpret_cast<const float4*>(rsk + c0);
+                const float tv = i & 2 ? (i & 1 ? thr[3] : thr[2]) : (i & 1 ? thr[1] : thr[0]);
+                uint32_t in = (fabsf(e.x * q.x) >= tv ? 1u : 0u) | (fabsf(e.y * q.y) >= tv ? 2u : 0u) | (fabsf(e.z * q.z) >= tv ? 4u : 0u) |
+                              (fabsf(e.w * q.w) >= tv ? 8u : 0u);
+                float b = 0.f;
+                while (in) {
+                    const int c = c0 + __ffs(in) - 1;
+                    in &= in - 1;
+                    b = fmaxf(b, fabsf(E[4 * i * 128 + c] / sk[c]));
+                }
+#pragma unroll
+                for (int n = 0; n < 4; ++n) best[n] = fmaxf(best[n], n == i ? b : 0.f);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
                 for (int i = 0; i < 4; ++i) best[i] = fmaxf(best[i], __shfl_xor_sync(0xffffffffu, best[i], o));
-            const float2 mg = make_float2(RNE_MAGIC, RNE_MAGIC);
+            const float2 mg = make_float2(RNE_MAGIC, RNE_MAGIC), neg = make_float2(-1.f, -1.f);
+            uint32_t tie = 0;                                          // rows with a value near a half-integer
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 best[i] = fmaxf(best[i], EPS);
@@ -361,12 +397,30 @@ quantize_kernel(lq_dims d, char* __restrict__ ssm, float* __restrict__ Wbuf, flo
                 if (l8 == 0) reinterpret_cast<float*>(base + CK_SV)[row0 + 4 * i] = best[i];
                 uint32_t* codes = reinterpret_cast<uint32_t*>(base + CK_CODES) + (row0 + 4 * i) * 32 + l8;
                 const float2 rv2 = make_float2(rv, rv);
+                float far = 0.f;                                       // from the nearest integer
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     // rint() by adding 1.5 * 2^23: the sum's low mantissa byte is the code in two's complement
                     const float2 x = a[i][2 * j], y = a[i][2 * j + 1];
                     const float2 tx = __ffma2_rn(x, rv2, mg), ty = __ffma2_rn(y, rv2, mg);
+                    const float2 dx = __ffma2_rn(x, rv2, __ffma2_rn(tx, neg, mg)), dy = __ffma2_rn(y, rv2, __ffma2_rn(ty, neg, mg));
                     codes[8 * j] = pack4(__float_as_uint(tx.x), __float_as_uint(tx.y), __float_as_uint(ty.x), __float_as_uint(ty.y));
+                    far = fmaxf(far, fmaxf(fmaxf(fabsf(dx.x), fabsf(dx.y)), fmaxf(fabsf(dy.x), fabsf(dy.y))));
+                }
+                tie |= far > 0.5f - TIE_BAND ? 1u << i : 0u;           // (one row of 500, or thereabouts, in a lane)
+            }
+            while (tie) {
+                const int i = __ffs(tie) - 1;
+                tie &= tie - 1;
+                const float sv = i & 2 ? (i & 1 ? best[3] : best[2]) : (i & 1 ? best[1] : best[0]), rf = QMAX / sv;
+#pragma unroll 1
+                for (int n = 0; n < 16; ++n) {
+                    const int c = 4 * l8 + 32 * (n >> 2) + (n & 3);
+                    const float e = E[4 * i * 128 + c], y = e * rsk[c] * rf;
+                    if (fabsf(y - rintf(y)) > 0.5f - 2.f * TIE_BAND) {
+                        const float z = e / (sk[c] * sv) * QMAX + RNE_MAGIC;
+                        reinterpret_cast<int8_t*>(base + CK_CODES)[(row0 + 4 * i) * 128 + c] = int8_t(__float_as_uint(z) & 0xffu);
+                    }
                 }
             }
             __syncwarp();                                              // every lane has read the last of the piece

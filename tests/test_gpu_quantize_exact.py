@@ -3,7 +3,8 @@ rounding of the first pass into codes of the second, so two builds that add in d
 
   factors   those of lq_lowrank on the transposed state, rounded to f16: sums of 64 + 64 products in index order, modified
             Gram-Schmidt by pairs (the two kernels share no code but that order)
-  scales    Sk = sqrt of the column means of |E| (64 + 64 rows in order)
+  scales    Sk = sqrt of the column means of |E| (64 + 64 rows in order), Sv = the largest true quotient |E / Sk| of a row
+  codes     rint(E / (Sk Sv) * 127) with true divisions
 """
 import numpy as np
 import pytest
@@ -78,6 +79,16 @@ def test_factor_bits(R, iters):
     # column scales: the same order of sums
     Sk = restated(S[1:].flatten(0, 1), want[..., :K], want[..., K:])[0]
     same("Sk", got["Sk"], Sk, kinds)
+
+
+@pytest.mark.gpu
+@CASES
+def test_scale_and_code_bits(R, iters):
+    S, kinds = heads(R, iters)
+    got = quantized(S, R, iters)
+    _, Sv, codes = restated(S[1:].flatten(0, 1), got["uq"][..., :K], got["uq"][..., K:])
+    same("Sv", got["Sv"], Sv, kinds)
+    same("Sq", got["Sq"], codes, kinds)
 
 
 @pytest.mark.gpu
