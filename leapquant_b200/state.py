@@ -98,7 +98,8 @@ class LeapQuantState:
         # launches are issued one by one from the host.
         self.conv_one_launch = False
         self._kconv = None
-        self._mixed = None
+        self._mixed = None                                    # activated rows of decode_conv
+        self._mixed_old = []                                  # smaller ones: a captured graph may hold their addresses
         # mailboxes for the heads whose window fills in a call (zeroed once, here): let a CTA without such a head take over a
         # head of a CTA that has several.  No counterpart in the reference.
         self.work = torch.zeros(KN.decode_work_ints(NS, HV), dtype=torch.int32, device=dev)
@@ -171,7 +172,10 @@ class LeapQuantState:
             if self._kconv is None:
                 self._kconv = KN.make_conv1d_update(self.NS, C)
             if self._mixed is None or self._mixed.shape[0] < N:
-                self._mixed = torch.empty(max(N, 64), C, dtype=torch.bfloat16, device=x.device)
+                # powers of two: the buffers kept for the graphs that hold them are together no larger than the newest one
+                if self._mixed is not None:
+                    self._mixed_old.append(self._mixed)
+                self._mixed = torch.empty(max(64, 1 << (N - 1).bit_length()), C, dtype=torch.bfloat16, device=x.device)
             mixed = self._mixed if self._mixed.shape[0] == N else self._mixed[:N]
             i32 = idx if idx.dtype == torch.int32 else idx.to(torch.int32)
             self._kconv(x, conv_state, conv_weight, conv_bias, i32, mixed)
