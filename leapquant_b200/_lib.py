@@ -119,10 +119,6 @@ raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getC
 current_device = torch._C._cuda_getDevice if hasattr(torch._C, "_cuda_getDevice") else torch.cuda.current_device
 
 
-def stream_of(t):
-    return raw_stream(t.get_device())
-
-
 def not_cuda():
     raise LeapQuantError("leapquant_b200 kernels take CUDA tensors only (there is no CPU fallback)")
 

@@ -140,12 +140,13 @@ class LeapQuantState:
         if idx.dtype != torch.int32:
             idx = idx.to(torch.int32)
         if self.fused:
-            q = ssm if ssm.dim() == 4 else self.views(ssm)["q32"]         # (the checkpoint begins where the fp32 slot does)
+            if ssm.dim() != 4:
+                raise ValueError(f"the state tensor is [slots, heads, V, K], got {tuple(ssm.shape)}")
             if self.kda:
-                self.kdecode(q, self.Kbuf, self.Ubuf, self.Wbuf, self.Pbuf, self.Gbuf, self.hcnt, mixed, a, b, A_log,
+                self.kdecode(ssm, self.Kbuf, self.Ubuf, self.Wbuf, self.Pbuf, self.Gbuf, self.hcnt, mixed, a, b, A_log,
                              dt_bias, self.Q0, idx, out, self.work)
             else:
-                self.kdecode(q, self.Kbuf, self.Ubuf, self.Wbuf, self.Pbuf, self.hcnt, mixed, a, b, A_log, dt_bias,
+                self.kdecode(ssm, self.Kbuf, self.Ubuf, self.Wbuf, self.Pbuf, self.hcnt, mixed, a, b, A_log, dt_bias,
                              self.Q0, idx, out, self.work)
             return
         v = self.views(ssm)
