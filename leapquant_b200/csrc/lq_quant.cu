@@ -175,8 +175,7 @@ quantize_kernel(lq_dims d, char* __restrict__ ssm, float* __restrict__ Wbuf, flo
                 *reinterpret_cast<float4*>(Qh + e) = make_float4(-round_f16(q.x), -round_f16(q.y), -round_f16(q.z), -round_f16(q.w));
             }
         };
-        // half steps: P = S^T Q, orthonormalised; Q = S P, orthonormalised; ...; U = S^T Q (one copy of each piece of code: a head
-        // runs through this loop body once from a cold instruction cache)
+        // half steps: P = S^T Q, orthonormalised; Q = S P, orthonormalised; ...; U = S^T Q (one copy of each piece of code)
 #pragma unroll 1
         for (int hs = 0;; ++hs) {
             const bool to_q = hs & 1, last = hs >= 2 * iters;
